@@ -8,7 +8,7 @@
 #include "ep_dstate.h"
 #include "ep_engine.h"
 #include "ep_kernels_impl.cuh"
-#include "ep_rfft.cuh"
+#include "ep_yz.cuh"
 
 #define EP_RED_BLOCKS 1216
 #define EP_SMEM_CAP (110 * 1024)
@@ -301,38 +301,21 @@ void Engine<T>::release() {
 }
 
 // ---------------------------------------------------------------------------
-// Register-resident transforms (ep_rfft.cuh) of lines of length N.
 #endif
 #if EP_ENGINE_PARTS & EP_PART_FFT
+// Launch of one of a length's Y / Z pass kernels (ep_yz.cuh) on n arrays or
+// convolution inputs.
 template <class T>
-template <int N>
-int Engine<T>::rfft_y(const Arr8<T>& a, int n, const LineSet& ls, int dir) {
-  dim3 grid((unsigned)((ls.nlines + 31) / 32), (unsigned)n), blk(32, rfft::Shape<N>::P);
-  const size_t sm = rfft::smem_bytes<T, N>();
-  if (dir < 0) {
-    auto k = k_c2c_r<T, N, -1>;
-    EP_LAUNCH("fft_y_fwd", k, grid, blk, sm, a, ls, twy);
-  } else {
-    auto k = k_c2c_r<T, N, +1>;
-    EP_LAUNCH("fft_y_inv", k, grid, blk, sm, a, ls, twy);
-  }
-  return EP_OK;
-}
-
-template <class T>
-template <int N>
-int Engine<T>::rfft_z(const ConvSpec<T>& cs, int nin, const LineSet& ls) {
-  dim3 grid((unsigned)((ls.nlines + 31) / 32), (unsigned)nin), blk(32, rfft::Shape<N>::P);
-  bool one = true;
-  for (int i = 0; i < nin; ++i) one = one && cs.nout[i] == 1;
-  if (one) {
-    auto k = k_zconv_r<T, N, true>;
-    EP_LAUNCH("fft_z_conv", k, grid, blk, (rfft::conv_smem_bytes<T, N, true>()), cs, ls, twz);
-  } else {
-    auto k = k_zconv_r<T, N, false>;
-    EP_LAUNCH("fft_z_conv", k, grid, blk, (rfft::conv_smem_bytes<T, N, false>()), cs, ls, twz);
-  }
-  return EP_OK;
+int Engine<T>::yz_launch(const char* name, const void* fn, const YZKernels& k, size_t smem, const LineSet& ls, int n,
+                         void** args) {
+  const dim3 grid((unsigned)((ls.nlines + k.lines - 1) / k.lines), (unsigned)n);
+  cudaEvent_t a = nullptr;
+  int c = -1;
+  prof->begin(st, name, a, c);
+  cudaError_t e = cudaLaunchKernel(fn, grid, dim3(k.threads), args, smem, st);
+  prof->end(st, c, a);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  return cuda_ok(e, name);
 }
 
 template <class T>
@@ -340,14 +323,12 @@ int Engine<T>::fft_y(CT** arrs, int n, int dir) {
   Arr8<T> a{};
   for (int i = 0; i < n; ++i) a.a[i] = arrs[i];
   LineSet ls{(long long)g.nxh, (long long)g.nxh * g.ny, (long long)g.nxh, (long long)g.nxh * g.nz};
-  switch (g.ny) {
-    case 32: return rfft_y<32>(a, n, ls, dir);
-    case 64: return rfft_y<64>(a, n, ls, dir);
-    case 128: return rfft_y<128>(a, n, ls, dir);
-    case 256: return rfft_y<256>(a, n, ls, dir);
-    case 96: if constexpr (sizeof(T) == 4) return rfft_y<96>(a, n, ls, dir); break;
-    case 192: if constexpr (sizeof(T) == 4) return rfft_y<192>(a, n, ls, dir); break;
-    default: break;
+  if (const YZKernels* k = yz_kernels<T>(g.ny)) {
+    const CT* tw = twy;
+    const int inverse = dir < 0 ? 0 : 1;
+    void* args[] = {&a, &ls, &tw};
+    return yz_launch(inverse ? "fft_y_inv" : "fft_y_fwd", k->c2c[inverse], *k, k->line_bytes + k->tw_bytes, ls, n,
+                     args);
   }
   const int LT = l_lines(g.ny, 2);
   dim3 grid((unsigned)((ls.nlines + LT - 1) / LT), (unsigned)n);
@@ -371,14 +352,12 @@ int Engine<T>::zconv(const CT* const* in, CT* const (*out)[3], const T* const (*
     for (int j = 0; j < nout[i]; ++j) { cs.out[i][j] = out[i][j]; cs.ker[i][j] = ker[i][j]; }
   }
   LineSet ls{(long long)g.nxh * g.ny, 0, (long long)g.nxh * g.ny, (long long)g.nxh * g.ny};
-  switch (g.nz) {
-    case 32: return rfft_z<32>(cs, nin, ls);
-    case 64: return rfft_z<64>(cs, nin, ls);
-    case 128: return rfft_z<128>(cs, nin, ls);
-    case 256: return rfft_z<256>(cs, nin, ls);
-    case 96: if constexpr (sizeof(T) == 4) return rfft_z<96>(cs, nin, ls); break;
-    case 192: if constexpr (sizeof(T) == 4) return rfft_z<192>(cs, nin, ls); break;
-    default: break;
+  if (const YZKernels* k = yz_kernels<T>(g.nz)) {
+    const CT* tw = twz;
+    int most = 1;
+    for (int i = 0; i < nin; ++i) most = std::max(most, nout[i]);
+    void* args[] = {&cs, &ls, &tw};
+    return yz_launch("fft_z_conv", k->conv, *k, (most > 1 ? 2 : 1) * k->line_bytes + k->tw_bytes, ls, nin, args);
   }
   const int LT = l_lines(g.nz, 3);
   dim3 grid((unsigned)((ls.nlines + LT - 1) / LT), (unsigned)nin);
@@ -387,9 +366,9 @@ int Engine<T>::zconv(const CT* const* in, CT* const (*out)[3], const T* const (*
   return EP_OK;
 }
 
-// First-derivative marches (k_d1march): mode 0 = grad f, mode 1 = dy f + dz f2.
 #endif
 #if EP_ENGINE_PARTS & EP_PART_MARCH
+// First-derivative marches (k_d1march): mode 0 = grad f, mode 1 = dy f + dz f2.
 template <class T>
 int Engine<T>::d1march(int mode, const T* f, const T* f2, T* o0, T* o1, T* o2) {
   dim3 grid((g.nx + EP_D1_TX - 1) / EP_D1_TX, (g.ny + EP_TY - 1) / EP_TY, (g.nz + zc_d1 - 1) / zc_d1);
@@ -1303,7 +1282,7 @@ int Engine<T>::autotune(std::string* report) {
     const int xreal[4] = {0, 4, 4, 1};
     for (int round = 0; round < 2; ++round) {
       for (int cls = 0; cls < 6; ++cls) {
-        if ((cls == 4 && rfft::supported<T>(g.ny)) || (cls == 5 && rfft::supported<T>(g.nz))) continue;
+        if ((cls == 4 && yz_kernels<T>(g.ny)) || (cls == 5 && yz_kernels<T>(g.nz))) continue;
         const Shapes keep = shp;
         Shapes bestS = shp;
         float best = cur;
@@ -1433,14 +1412,11 @@ int Engine<T>::fft_attrs() {
   cudaFuncSetAttribute(k_c2c<T, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(k_c2c<T, +1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(k_zconv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-#define EP_RFFT_ATTR(NN)                                                                                  \
-  cudaFuncSetAttribute(k_c2c_r<T, NN, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rfft::smem_bytes<T, NN>()); \
-  cudaFuncSetAttribute(k_c2c_r<T, NN, +1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rfft::smem_bytes<T, NN>()); \
-  cudaFuncSetAttribute(k_zconv_r<T, NN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rfft::conv_smem_bytes<T, NN, true>()); \
-  cudaFuncSetAttribute(k_zconv_r<T, NN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rfft::conv_smem_bytes<T, NN, false>());
-  EP_RFFT_ATTR(32) EP_RFFT_ATTR(64) EP_RFFT_ATTR(128) EP_RFFT_ATTR(256)
-  if constexpr (sizeof(T) == 4) { EP_RFFT_ATTR(96) EP_RFFT_ATTR(192) }
-#undef EP_RFFT_ATTR
+  if (const YZKernels* k = yz_kernels<T>(g.ny))
+    for (const void* f : k->c2c)
+      cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(k->line_bytes + k->tw_bytes));
+  if (const YZKernels* k = yz_kernels<T>(g.nz))
+    cudaFuncSetAttribute(k->conv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * k->line_bytes + k->tw_bytes));
   return EP_OK;
 }
 #endif

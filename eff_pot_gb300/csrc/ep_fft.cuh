@@ -110,6 +110,7 @@ template <class T, int R, int DIR> EP_DEV void dftR(C2<T>* v) {
   else if (R == 5) dft5<T, DIR>(v);
   else dft8<T, DIR>(v);
 }
+template <class T, int R, int DIR> EP_DEV void dft(C2<T>* v);
 
 template <class T> struct K16;
 template <> struct K16<double> {
@@ -226,7 +227,7 @@ EP_DEV void tw_ab(C2<T>* y) {
   }
 }
 
-// N = A B point DFT (A, B in {2, 3, 4, 5, 8}) in registers:
+// N = A B point DFT (A, B any length of dft) in registers:
 //   n = B n1 + n2, k = k1 + A k2,
 //   X[k1 + A k2] = sum_n2 w_B^(n2 k2) w_N^(n2 k1) sum_n1 x[B n1 + n2] w_A^(n1 k1)
 template <class T, int A, int B, int DIR> EP_DEV void dft_ab(C2<T>* v) {
@@ -237,7 +238,7 @@ template <class T, int A, int B, int DIR> EP_DEV void dft_ab(C2<T>* v) {
     C2<T> a[A];
 #pragma unroll
     for (int n1 = 0; n1 < A; ++n1) a[n1] = v[B * n1 + n2];
-    dftR<T, A, DIR>(a);
+    dft<T, A, DIR>(a);
 #pragma unroll
     for (int k1 = 0; k1 < A; ++k1) y[A * n2 + k1] = a[k1];
   }
@@ -247,23 +248,26 @@ template <class T, int A, int B, int DIR> EP_DEV void dft_ab(C2<T>* v) {
     C2<T> b[B];
 #pragma unroll
     for (int n2 = 0; n2 < B; ++n2) b[n2] = y[A * n2 + k1];
-    dftR<T, B, DIR>(b);
+    dft<T, B, DIR>(b);
 #pragma unroll
     for (int k2 = 0; k2 < B; ++k2) v[k1 + A * k2] = b[k2];
   }
 }
 
-// Register DFT of R points, R in {2, 4, 8, 12, 16, 20, 24}.
+// Register DFT of R points, R in {2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16, 18, 20, 24}.
 template <class T, int R, int DIR> EP_DEV void dft(C2<T>* v) {
   if constexpr (R == 16) dft16<T, DIR>(v);
-  else if constexpr (R == 8) dft8<T, DIR>(v);
-  else if constexpr (R == 4) dft4<T, DIR>(v);
+  else if constexpr (R == 6) dft_ab<T, 3, 2, DIR>(v);
+  else if constexpr (R == 9) dft_ab<T, 3, 3, DIR>(v);
+  else if constexpr (R == 10) dft_ab<T, 5, 2, DIR>(v);
   else if constexpr (R == 12) dft_ab<T, 4, 3, DIR>(v);
+  else if constexpr (R == 15) dft_ab<T, 5, 3, DIR>(v);
+  else if constexpr (R == 18) dft_ab<T, 9, 2, DIR>(v);
   else if constexpr (R == 20) dft_ab<T, 4, 5, DIR>(v);
   else if constexpr (R == 24) dft_ab<T, 8, 3, DIR>(v);
   else {
-    static_assert(R == 2, "register DFT length");
-    dft2<T, DIR>(v);
+    static_assert(R == 2 || R == 3 || R == 4 || R == 5 || R == 8, "register DFT length");
+    dftR<T, R, DIR>(v);
   }
 }
 

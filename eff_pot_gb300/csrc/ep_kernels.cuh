@@ -202,7 +202,7 @@ EP_DEV T hexp_t(const Phys& ph, C2<T> psi, C2<T> H) {
 // Half-line transforms of N2 = nx/2 points.  N2 in {16, 32, 64, 128} (and
 // in FP32 also 48, 80, 96) use
 // xlines: P threads of one warp per line, E = N2/P points per thread, the
-// two-factor decomposition of ep_rfft.cuh with the exchange done in place in
+// two-factor decomposition of ep_yz.cuh with the exchange done in place in
 // the line's own shared-memory row (stride P+1 for the exchange), fenced by
 // __syncwarp only.  The row stride x_row() makes the step-1 reads, the
 // exchange and the step-2 reads conflict-free for 8- and 16-byte elements.
