@@ -495,6 +495,7 @@ int ep_destroy(ep_ctx* c) {
   if (c->imp.d_potpi) cudaFree(c->imp.d_potpi);
   if (c->imp.d_potdel) cudaFree(c->imp.d_potdel);
   if (c->imp.d_potsigdel) cudaFree(c->imp.d_potsigdel);
+  if (c->imp.d_coef) cudaFree(c->imp.d_coef);
   if (c->imp.d_potpi_f) cudaFree(c->imp.d_potpi_f);
   if (c->imp.d_potdel_f) cudaFree(c->imp.d_potdel_f);
   c->prof.release();
@@ -536,45 +537,69 @@ int ep_set_impurity_potentials(ep_ctx* c, const ep_potential* pi, const ep_poten
   return ep_set_impurity_tables(c, tp.data(), td.data(), npot, del, sigma->umax);
 }
 
-// Replaces the device tables (d_potpi, d_potdel, d_potsigdel) by tabs[0..2]
-// (NULL: none) of npot + 2 entries each.
-static int upload_tables(ep_ctx* c, const double* const tabs[3], int npot) {
+// The parabolas of update() (potenimp.f90:588-632) through f(i0-1), f(i0),
+// f(i0+1) for every i0 and for both of its branches (r below the node i0 first,
+// then above), with its coefficients aa, bb, cc of r: entries at
+// ((branch * (npot + 2) + i0) * 8 + at).
+static void parabolas(const double* f, int npot, double h, int at, std::vector<double>& coef) {
+  const double c1oh = 1.0 / h, c1o2h2 = c1oh * c1oh * 0.5;
+  for (int branch = 0; branch < 2; ++branch) {
+    for (int i0 = 1; i0 <= npot; ++i0) {
+      const bool lo = branch == 0;
+      const double r0 = (i0 - 1) * h, f0 = f[i0], f1 = f[lo ? i0 - 1 : i0 + 1], f2 = f[lo ? i0 + 1 : i0 - 1];
+      const double aa = (f2 - 2.0 * f0 + f1) * c1o2h2;
+      const double bb = ((lo ? f2 : f1) - f0) * c1oh - aa * (2.0 * r0 + h);
+      double* o = coef.data() + ((size_t)branch * (npot + 2) + i0) * 8 + at;
+      o[0] = aa;
+      o[1] = bb;
+      o[2] = f0 - r0 * (bb + r0 * aa);
+    }
+  }
+}
+
+// Replaces the device tables by tabs[0..2] (NULL: none) of npot + 2 entries
+// each: in the D state d_potpi, d_potdel, d_potsigdel; in the P state the
+// parabolas of tabs[0] and tabs[1] and their FP32 copies.
+static int upload_tables(ep_ctx* c, const double* const tabs[3], int npot, double delinter) {
   cudaSetDevice(c->cfg.device);
-  double** dst[3] = {&c->imp.d_potpi, &c->imp.d_potdel, &c->imp.d_potsigdel};
+  ImpState& m = c->imp;
+  double** dst[4] = {&m.d_potpi, &m.d_potdel, &m.d_potsigdel, &m.d_coef};
   for (double** d : dst) {
     if (*d) cudaFree(*d);
     *d = nullptr;
   }
-  float** dstf[2] = {&c->imp.d_potpi_f, &c->imp.d_potdel_f};
+  float** dstf[2] = {&m.d_potpi_f, &m.d_potdel_f};
   for (float** d : dstf) {
     if (*d) cudaFree(*d);
     *d = nullptr;
   }
-  c->imp.have_tables = false;
-  const size_t n = (size_t)(npot + 2) * sizeof(double);
-  for (int i = 0; i < 3; ++i) {
-    if (!tabs[i]) continue;
-    if (cudaMalloc((void**)dst[i], n) != cudaSuccess) {
+  m.have_tables = false;
+  auto put = [&](void** d, const void* h, size_t n) -> int {
+    if (cudaMalloc(d, n) != cudaSuccess) {
       cudaGetLastError();
-      *dst[i] = nullptr;
+      *d = nullptr;
       return fail(c, EP_ERR_OOM, "table allocation failed");
     }
-    cudaMemcpyAsync(*dst[i], tabs[i], n, cudaMemcpyHostToDevice, c->st);
-  }
-  // P state: FP32 copies for the FP32 engine's field evaluation
-  std::vector<float> tf((size_t)npot + 2);
-  for (int i = 0; i < 2 && c->cfg.state == EP_STATE_P; ++i) {
-    for (size_t k = 0; k < tf.size(); ++k) tf[k] = (float)tabs[i][k];
-    if (cudaMalloc((void**)dstf[i], tf.size() * sizeof(float)) != cudaSuccess) {
-      cudaGetLastError();
-      *dstf[i] = nullptr;
-      return fail(c, EP_ERR_OOM, "table allocation failed");
-    }
-    if (cudaMemcpy(*dstf[i], tf.data(), tf.size() * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess)
+    if (cudaMemcpy(*d, h, n, cudaMemcpyHostToDevice) != cudaSuccess)
       return fail(c, EP_ERR_CUDA, "table upload failed");
+    return EP_OK;
+  };
+  const size_t n = (size_t)npot + 2;
+  int r;
+  if (c->cfg.state == EP_STATE_D) {
+    for (int i = 0; i < 3; ++i)
+      if (tabs[i] && (r = put((void**)dst[i], tabs[i], n * sizeof(double)))) return r;
+    return EP_OK;
   }
-  if (cudaStreamSynchronize(c->st) != cudaSuccess) return fail(c, EP_ERR_CUDA, "table upload failed");
-  return EP_OK;
+  const double rmax = (npot - 1) * delinter, h = rmax / (npot - 1);
+  std::vector<double> coef(2 * n * 8, 0.0);
+  std::vector<float> tf(n);
+  for (int i = 0; i < 2; ++i) {
+    parabolas(tabs[i], npot, h, 3 * i, coef);
+    for (size_t k = 0; k < n; ++k) tf[k] = (float)tabs[i][k];
+    if ((r = put((void**)dstf[i], tf.data(), n * sizeof(float)))) return r;
+  }
+  return put((void**)&m.d_coef, coef.data(), coef.size() * sizeof(double));
 }
 
 int ep_set_impurity_tables(ep_ctx* c, const double* potpi, const double* potdel, int npot, double delinter,
@@ -582,7 +607,7 @@ int ep_set_impurity_tables(ep_ctx* c, const double* potpi, const double* potdel,
   if (!c || !potpi || !potdel || npot < 3 || !(delinter > 0)) return EP_ERR_INVALID_ARG;
   if (c->cfg.state != EP_STATE_P) return fail(c, EP_ERR_STATE, "D state: use ep_set_impurity_tables_d");
   const double* tabs[3] = {potpi, potdel, nullptr};
-  int r = upload_tables(c, tabs, npot);
+  int r = upload_tables(c, tabs, npot, delinter);
   if (r) return r;
   c->imp.npot = npot;
   c->imp.delinter = delinter;
@@ -623,7 +648,7 @@ int ep_set_impurity_tables_d(ep_ctx* c, const double* potdel, const double* potp
   if (!c || !potdel || !potpidel || !potsigdel || npot < 3 || !(delinter > 0)) return EP_ERR_INVALID_ARG;
   if (c->cfg.state != EP_STATE_D) return fail(c, EP_ERR_STATE, "D-state tables need state = EP_STATE_D");
   const double* tabs[3] = {potpidel, potdel, potsigdel};
-  int r = upload_tables(c, tabs, npot);
+  int r = upload_tables(c, tabs, npot, delinter);
   if (r) return r;
   c->imp.npot = npot;
   c->imp.delinter = delinter;

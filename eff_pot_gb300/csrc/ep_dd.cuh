@@ -111,6 +111,42 @@ EP_HD dfloat sqrt(dfloat a) {
   return dd_fast2sum(r, d.hi / (2.0f * r));
 }
 
+// exp(x) to about 2^-37: x = n ln 2 + r with |r| <= 0.35 (ln 2 in three FP32
+// parts, the products by the FMA error), then 1 + r + r^2 (1/2 + r (1/6 + r
+// (1/24 + ..))) by its Taylor series to r^11, the terms above r^4 in FP32 (below
+// 4e-12 of the result), and the power of two in two factors (results under the
+// FP32 range go to zero).
+EP_HD dfloat dd_exp(dfloat x) {
+  if (!(x.hi < 89.0f)) return dfloat(x.hi * 1e38f, 0.0f);  // overflow, NaN
+  if (x.hi < -104.0f) return dfloat(0.0f, 0.0f);
+  const float n = rintf(x.hi * 1.4426950408889634f);
+  // ln 2 = 0x1.62e4p-1 (15 bits: n times it is exact) + two FP32 remainders
+  const float l1 = 0.693145751953125f, l2 = 1.4286068e-06f, l3 = 5.497923e-14f;
+  dfloat r = dd_two_sum(EP_DD_FMA(-n, l1, x.hi), x.lo);
+  const float p2 = EP_DD_MUL(n, l2);
+  r = r - dfloat(p2, EP_DD_FMA(n, l3, EP_DD_FMA(n, l2, -p2)));
+  const float h = r.hi;
+  float t = 2.5052108e-8f;                 // 1/11!
+  t = EP_DD_FMA(t, h, 2.7557319e-7f);      // 1/10!
+  t = EP_DD_FMA(t, h, 2.7557319e-6f);      // 1/9!
+  t = EP_DD_FMA(t, h, 2.4801587e-5f);      // 1/8!
+  t = EP_DD_FMA(t, h, 1.9841270e-4f);      // 1/7!
+  t = EP_DD_FMA(t, h, 1.3888889e-3f);      // 1/6!
+  t = EP_DD_FMA(t, h, 8.3333333e-3f);      // 1/5!
+  dfloat p = dfloat(1.0 / 24.0) + r * dfloat(t, 0.0f);
+  p = dfloat(1.0 / 6.0) + r * p;
+  p = dfloat(0.5) + r * p;
+  p = r + (r * r) * p;
+  p = dfloat(1.0f, 0.0f) + p;
+  const int n1 = (int)n / 2, n2 = (int)n - n1;
+#if defined(__CUDA_ARCH__)
+  const float s1 = __int_as_float((n1 + 127) << 23), s2 = __int_as_float((n2 + 127) << 23);
+#else
+  const float s1 = ldexpf(1.0f, n1), s2 = ldexpf(1.0f, n2);
+#endif
+  return dfloat(p.hi * s1 * s2, p.lo * s1 * s2);
+}
+
 #if defined(__CUDACC__)
 __device__ __forceinline__ dfloat __shfl_sync(unsigned m, dfloat v, int src) {
   return dfloat(__shfl_sync(m, v.hi, src), __shfl_sync(m, v.lo, src));
@@ -124,6 +160,10 @@ __device__ __forceinline__ dfloat __shfl_xor_sync(unsigned m, dfloat v, int d) {
 __device__ __forceinline__ dfloat __ldg(const dfloat* p) {
   const float2 v = __ldg(reinterpret_cast<const float2*>(p));
   return dfloat(v.x, v.y);
+}
+__device__ __forceinline__ dfloat2 __ldg(const dfloat2* p) {
+  const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+  return dfloat2{dfloat(v.x, v.y), dfloat(v.z, v.w)};
 }
 __device__ __forceinline__ dfloat __ldcg(const dfloat* p) {
   const float2 v = __ldcg(reinterpret_cast<const float2*>(p));

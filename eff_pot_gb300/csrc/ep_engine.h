@@ -12,6 +12,7 @@
 #include "ep_kernels.cuh"
 
 struct YZKernels;
+struct ColGrid;
 
 // Launch accounting and optional per-class event timing.
 struct Prof {
@@ -42,14 +43,16 @@ struct ImpState {
   double pcr[3] = {0, 0, 0}, pcv[3] = {0, 0, 0};
   std::complex<double> qiv[10], invarold[10][3], hinvarold[10][2], pciv[10];
   // interpolation tables (module interpol), FP64 on the device
-  // P state: d_potpi = V_Pi, d_potdel = V_Sigma - V_Pi.  D state:
-  // d_potdel = V_Delta, d_potpi = V_Pi - V_Delta, d_potsigdel = V_Sigma - V_Delta.
+  // P state: d_coef, the parabolas of V_Pi and V_Sigma - V_Pi per interval and
+  // side (ImpTable).  D state: d_potdel = V_Delta, d_potpi = V_Pi - V_Delta,
+  // d_potsigdel = V_Sigma - V_Delta.
   int npot = 0;
   double delinter = 0, umax_sigma = 9.674836e3, umax_pi = 0.0;
   double* d_potpi = nullptr;
   double* d_potdel = nullptr;
   double* d_potsigdel = nullptr;
-  // P state: FP32 copies of d_potpi, d_potdel for the FP32 engine
+  double* d_coef = nullptr;
+  // P state: FP32 copies of V_Pi, V_Sigma - V_Pi for the FP32 engine
   float* d_potpi_f = nullptr;
   float* d_potdel_f = nullptr;
   ep_potential plus{};  // series pointer cleared: the fit lives in plus_series
@@ -227,6 +230,7 @@ class Engine {
   int rk_stage(int jr, double dt);
   int reduce_finalize(int nblocks, int nq, int out0, int mode);
   int read_sums(double* h, int n, int off);
+  dim3 col_grid(ColGrid& cg) const;
   int fft_y(CT** arrs, int n, int dir);
   int yz_launch(const char* name, const void* fn, const YZKernels& k, size_t smem, const LineSet& ls, int n,
                 void** args);

@@ -475,28 +475,51 @@ int Engine<T>::potenimp() {
       float2 fv[6];
       for (int i = 0; i < 6; ++i) fv[i] = make_float2((float)imp->invar[i].real(), (float)imp->invar[i].imag());
       const double h = rmax / (imp->npot - 1);
+      ColGrid cg;
+      const dim3 grid = col_grid(cg);
       auto kf = k_potenimp_f;
-      EP_LAUNCH("potenimp", kf, 4 * 152, 256, 0, g, (float)cfg.xmax, (float)cfg.ymax, (float)cfg.zmax, (float)hx,
-                (float)hy, (float)hz, (float)imp->rimp[0], (float)imp->rimp[1], (float)imp->rimp[2], imp->d_potpi_f,
+      EP_LAUNCH("potenimp", kf, grid, dim3(32, 8), cg.rows * sizeof(float), g, cg, cfg.xmax, cfg.ymax, cfg.zmax, hx,
+                hy, hz, imp->rimp[0], imp->rimp[1], imp->rimp[2], imp->d_potpi_f,
                 imp->d_potdel_f, imp->npot, (float)h, (float)(1.0 / h), (float)imp->umax_sigma, fv[0], fv[1], fv[2],
                 fv[3], fv[4], fv[5], vpi, delta, uimp);
       return EP_OK;
     }
   }
-  double2 iv[6];
-  for (int i = 0; i < 6; ++i) iv[i] = make_double2(imp->invar[i].real(), imp->invar[i].imag());
-  auto k = k_potenimp<T>;
-  EP_LAUNCH("potenimp", k, 4 * 152, 256, 0, g, cfg.xmax, cfg.ymax, cfg.zmax, hx, hy, hz, imp->rimp[0],
-            imp->rimp[1], imp->rimp[2], imp->d_potpi, imp->d_potdel, imp->npot, rmax, imp->umax_sigma, iv[0], iv[1],
-            iv[2], iv[3], iv[4], iv[5], vpi, delta, uimp);
+  if constexpr (sizeof(T) == 8) {
+    double2 iv[6];
+    for (int i = 0; i < 6; ++i) iv[i] = make_double2(imp->invar[i].real(), imp->invar[i].imag());
+    const double h = rmax / (imp->npot - 1);
+    const ImpTable tab{imp->d_coef, imp->npot, h, 1.0 / h, imp->umax_sigma};
+    ColGrid cg;
+    const dim3 grid = col_grid(cg);
+    auto k = k_potenimp<T>;
+    EP_LAUNCH("potenimp", k, grid, dim3(32, 8), cg.rows * sizeof(double2), g, cg, cfg.xmax, cfg.ymax, cfg.zmax, hx, hy, hz, imp->rimp[0],
+              imp->rimp[1], imp->rimp[2], tab, iv[0], iv[1], iv[2], iv[3], iv[4], iv[5], vpi, delta, uimp);
+  }
   return EP_OK;
+}
+
+// Launch grid of the column kernels: groups of 32 columns by chunks of rows,
+// at least three CTAs per SM where the grid allows (an FP64-bound kernel of
+// 160 CTAs would leave 144 SMs idle for half its time), at most EP_RED_BLOCKS
+// in all, the groups spread evenly over the CTAs of a chunk.
+template <class T>
+dim3 Engine<T>::col_grid(ColGrid& cg) const {
+  cg.groups = (int)(((long long)g.nx * g.nz + 31) / 32);
+  int chunks = (3 * dev_sm + cg.groups - 1) / cg.groups;
+  chunks = std::max(1, std::min(chunks, g.ny / 8));
+  chunks = std::max(chunks, (g.ny + 2047) / 2048);  // the row tables: 16 bytes a row at most
+  cg.rows = (g.ny + chunks - 1) / chunks;
+  chunks = (g.ny + cg.rows - 1) / cg.rows;
+  const int most = std::max(1, EP_RED_BLOCKS / chunks);
+  const int rounds = (cg.groups + most - 1) / most;
+  return dim3((unsigned)((cg.groups + rounds - 1) / rounds), (unsigned)chunks);
 }
 
 template <class T>
 int Engine<T>::reduce_finalize(int nblocks, int nq, int out0, int mode) {
   auto k = k_finalize;
-  const int renorm = (cfg.time_mode == EP_IMAGINARY_TIME && cfg.renormalize) ? 1 : 0;
-  EP_LAUNCH("finalize", k, 1, 256, 0, partials, nblocks, nq, sc, out0, mode, (double)g.N, dxyz, cfg.n4, renorm);
+  EP_LAUNCH("finalize", k, nq, 128, 0, partials, nblocks, nq, sc, out0, mode, dxyz, cfg.n4);
   return EP_OK;
 }
 
@@ -518,14 +541,28 @@ int Engine<T>::energy(ep_energies* e) {
   vp.umax = imp->plus.umax;
   for (int i = 0; i < 4; ++i) vp.par[i] = imp->plus.par[i];
   vp.s = imp->plus_series;
-  auto k = k_energy<T>;
-  EP_LAUNCH("energy", k, EP_RED_BLOCKS, 256, 0, g, fd, phys, psi, den, dencg, delj4, falfs, dxd, dyd, dzd, intx,
-            inty, intz, uimp, cfg.xmax, cfg.ymax, cfg.zmax, hx, hy, hz, imp->rimp[0], imp->rimp[1], imp->rimp[2],
-            cfg.z_exciplex_exclusion, vp, cfg.impurity != EP_IMPURITY_NONE ? 1 : 0, partials);
-  int r;
-  if ((r = reduce_finalize(EP_RED_BLOCKS, 8, 8, 0))) return r;
+  ColGrid cg;
+  const dim3 grid = col_grid(cg);
   double s[8];
-  if ((r = read_sums(s, 8, 8))) return r;
+  // W: the arithmetic of the terms (k_energy); mode 3 leaves the flag alone
+  auto sums = [&](auto w, int mode) -> int {
+    auto k = k_energy<T, decltype(w)>;
+    EP_LAUNCH("energy", k, grid, dim3(32, 8), cg.rows * sizeof(dfloat), g, cg, fd, phys, psi, den, dencg, delj4, falfs, dxd, dyd, dzd, intx,
+              inty, intz, uimp, cfg.xmax, cfg.ymax, cfg.zmax, hx, hy, hz, imp->rimp[0], imp->rimp[1], imp->rimp[2],
+              cfg.z_exciplex_exclusion, vp, cfg.impurity != EP_IMPURITY_NONE ? 1 : 0, partials);
+    int r = reduce_finalize((int)(grid.x * grid.y), 8, 8, mode);
+    return r ? r : read_sums(s, 8, 8);
+  };
+  int r;
+  if constexpr (std::is_same<T, double>::value) {
+    if ((r = sums(double(), 0))) return r;
+  } else {
+    if ((r = sums(dfloat(), 3))) return r;
+    bool fine = true;
+    for (double v : s) fine = fine && std::isfinite(v);
+    // beyond the FP32 range of the pairs (a diverging state): FP64 terms
+    if (!fine && (r = sums(double(), 0))) return r;
+  }
   const ep_config& c = cfg;
   e->ekin4 = c.h2o2m4 * s[0] * dxyz;
   e->elj4 = 0.5 * s[1] * dxyz;
@@ -595,18 +632,13 @@ int Engine<T>::forceimp(double* F) {
     for (int i = 0; i < 3; ++i) F[i] = -s[i] * dxyz;
     return EP_OK;
   }
-  if constexpr (sizeof(T) == 4) {
-    auto kf = k_impmoments_f;
-    EP_LAUNCH("impmoments", kf, EP_RED_BLOCKS, 256, 0, g, den, dxd, dyd, dzd, uimp, vpi, delta, (float)cfg.xmax,
-              (float)cfg.ymax, (float)cfg.zmax, (float)hx, (float)hy, (float)hz, (float)imp->rimp[0],
-              (float)imp->rimp[1], (float)imp->rimp[2], izlo, izhi, partials);
-  } else {
-    auto k = k_impmoments<T>;
-    EP_LAUNCH("impmoments", k, EP_RED_BLOCKS, 256, 0, g, den, dxd, dyd, dzd, uimp, vpi, delta, cfg.xmax, cfg.ymax,
-              cfg.zmax, hx, hy, hz, imp->rimp[0], imp->rimp[1], imp->rimp[2], izlo, izhi, partials);
-  }
+  ColGrid cg;
+  const dim3 grid = col_grid(cg);
+  auto k = k_impmoments<T>;
+  EP_LAUNCH("impmoments", k, grid, dim3(32, 8), cg.rows * sizeof(T), g, cg, den, dxd, dyd, dzd, uimp, vpi, delta,
+            cfg.xmax, cfg.ymax, cfg.zmax, hx, hy, hz, imp->rimp[0], imp->rimp[1], imp->rimp[2], izlo, izhi, partials);
   int r;
-  if ((r = reduce_finalize(EP_RED_BLOCKS, 9, 16, 0))) return r;
+  if ((r = reduce_finalize((int)(grid.x * grid.y), 9, 16, 0))) return r;
   double s[9];
   if ((r = read_sums(s, 9, 16))) return r;
   for (int i = 0; i < 3; ++i) F[i] = -s[i] * dxyz;

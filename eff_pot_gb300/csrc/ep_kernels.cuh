@@ -1839,19 +1839,10 @@ __global__ void k_materialize(SlotPtrs<T> bufs, T* __restrict__ den, long long N
 __global__ void k_reset_scales(DevScalars* sc);
 
 // Sum of partials (fixed order, compensated) -> sc->sums[out0 + q].
-// mode 1: corrector epilogue (errHe, norm, mu, renormalisation factor).
-// mode 2: norm only (renormalisation factor).
+// one CTA per sum.  mode 2: the sum is the norm (renormalisation factor);
+// mode 3: a sum that is not finite raises no flag.
 __global__ void k_finalize(const double* __restrict__ partials, int nblocks, int nq, DevScalars* sc, int out0,
-                           int mode, double N, double dxyz, double n4, int renorm);
-
-// Impurity field: updatepoten + potenimp P state (potenimp.f90:1-46,184-186,
-// 515-632).  Tables are FP64 (0..npot+1).
-template <class T>
-__global__ void k_potenimp(Geo g, double xmax, double ymax, double zmax, double hx, double hy, double hz,
-                           double r0, double r1, double r2, const double* __restrict__ potpi,
-                           const double* __restrict__ potdel, int npot, double rmax, double umax_sigma,
-                           double2 iv0, double2 iv1, double2 iv2, double2 iv3, double2 iv4, double2 iv5,
-                           T* __restrict__ vpi, T* __restrict__ delta, T* __restrict__ uimp);
+                           int mode, double dxyz, double n4);
 
 // D state (potenimp.f90:47-182, 545-566): Delta = V_Delta(r),
 // Pi_Del = (V_Pi - V_Delta)(r)/r^4, Sig_Del = (V_Sigma - V_Delta)(r)/r^4 and
@@ -1875,24 +1866,6 @@ struct PotDev {
   double r_cutoff, umax, par[4];
   ep_series s;  // EP_POT_SERIES
 };
-template <class T>
-__global__ void k_energy(Geo g, FdW<T> fd, Phys ph, const C2<T>* __restrict__ psi, const T* __restrict__ den,
-                         const T* __restrict__ dencg, const T* __restrict__ delj4, const T* __restrict__ falfs,
-                         const T* __restrict__ dxd, const T* __restrict__ dyd, const T* __restrict__ dzd,
-                         const T* __restrict__ ix, const T* __restrict__ iy, const T* __restrict__ iz,
-                         const T* __restrict__ uimp, double xmax, double ymax, double zmax, double hx, double hy,
-                         double hz, double r0, double r1, double r2, double zexc, const __grid_constant__ PotDev vplus,
-                         int impurity, double* __restrict__ partials);
-
-// forceimp / potinvar moments (potenimp.f90:193-258, 298-317); the F_z sum
-// runs over the planes izlo <= iz < izhi (the exciplex filter, :211-248).
-template <class T>
-__global__ void k_impmoments(Geo g, const T* __restrict__ den, const T* __restrict__ dxd,
-                             const T* __restrict__ dyd, const T* __restrict__ dzd, const T* __restrict__ uimp,
-                             const T* __restrict__ vpi, const T* __restrict__ delta, double xmax, double ymax,
-                             double zmax, double hx, double hy, double hz, double r0, double r1, double r2,
-                             int izlo, int izhi, double* __restrict__ partials);
-
 // forceimp sums + the D-state matrix (potenimp.f90:331-405): 3 + 15 sums,
 // the matrix's upper triangle in DGram's order.
 template <class T>

@@ -46,29 +46,132 @@ EP_DEV double pot_eval(const PotDev& v, double r) {
   return ep_pair_potential(v.kind, v.r_cutoff, v.umax, v.par, &v.s, r);
 }
 
-template <class T>
-__global__ void k_potenimp(Geo g, double xmax, double ymax, double zmax, double hx, double hy, double hz,
-                           double r0, double r1, double r2, const double* __restrict__ potpi,
-                           const double* __restrict__ potdel, int npot, double rmax, double umax_sigma,
-                           double2 iv0, double2 iv1, double2 iv2, double2 iv3, double2 iv4, double2 iv5,
-                           T* __restrict__ vpi, T* __restrict__ delta, T* __restrict__ uimp) {
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < g.N; p += (long long)gridDim.x * blockDim.x) {
-    int ix, iy, iz;
-    idx3(g, p, ix, iy, iz);
-    const double xx = coord(xmax, hx, ix) - r0;
-    const double yy = coord(ymax, hy, iy) - r1;
-    const double zz = coord(zmax, hz, iz) - r2;
-    const double rr2 = rr2_nc(xx, yy, zz);
-    const double r = sqrt(rr2);
-    const double vp = interp_update(r, npot, rmax, potpi);
-    const double dl = r > 1e-3 ? interp_update(r, npot, rmax, potdel) / rr2 : umax_sigma;
-    const double ox = iv0.x * xx + iv2.x * yy + iv4.x * zz, oy = iv0.y * xx + iv2.y * yy + iv4.y * zz;
-    const double ex = iv1.x * xx + iv3.x * yy + iv5.x * zz, ey = iv1.y * xx + iv3.y * yy + iv5.y * zz;
-    const double u = vp + dl * ((ox * ox + oy * oy) + (ex * ex + ey * ey));
-    vpi[p] = (T)vp;
-    delta[p] = (T)dl;
-    uimp[p] = (T)fmin(u, 1000.0);
+// Column mapping of the impurity and energy kernels: a warp takes 32
+// neighbouring (x, z) columns and its block's warps share the rows y of the
+// block's chunk, so the coordinates x and z (and what depends on them alone)
+// are per column instead of per point, no point needs an index division, and
+// the neighbour rows a gradient reads are shared by the block's warps.
+// setup(x index, z index, offset of (x, 0, z)) opens a column; body(y index,
+// offset) takes a point; done() closes the column.  Blocks are 32 x 8 threads;
+// UNROLL rows are in flight at once.
+struct ColGrid {
+  int groups;  // groups of 32 columns
+  int rows;    // rows of a y chunk (blockIdx.y)
+};
+template <int UNROLL = 1, class Setup, class Body, class Done>
+EP_DEV void columns(const Geo& g, const ColGrid& cg, Setup&& setup, Body&& body, Done&& done) {
+  const int ncol = g.nx * g.nz;
+  const int y0 = blockIdx.y * cg.rows, y1 = min(y0 + cg.rows, g.ny);
+  for (int grp = blockIdx.x; grp < cg.groups; grp += gridDim.x) {
+    const int col = grp * 32 + (int)threadIdx.x;
+    if (col < ncol) {
+      const int iz = col / g.nx, ix = col - iz * g.nx;
+      const long long p0 = ix + (long long)g.nx * g.ny * iz;
+      setup(ix, iz, p0);
+#pragma unroll UNROLL
+      for (int iy = y0 + (int)threadIdx.y; iy < y1; iy += 8) body(iy, p0 + (long long)g.nx * iy);
+      done();
+    }
   }
+}
+
+// V_Pi and the P-state Delta of updatepoten at |x - r_imp|^2 = rr2, from the
+// parabolas of update() (potenimp.f90:588-632) tabulated per interval and side
+// (upload_tables).  r and 1 / r^2 come from one reciprocal square root with a
+// correction of r; where r / h falls within 1e-5 of a switch of the parabola
+// (the next interval, or the other side of a node), r <= 1e-3 or the table's
+// end, the root and the quotients are taken as update() takes them, so the
+// interval is the one it takes.
+struct ImpTable {
+  const double* coef;  // [2][npot + 2][8]: aa, bb, cc of V_Pi, then of V_Sigma - V_Pi
+  int npot;
+  double h, rh;        // spacing and its reciprocal
+  double umax_sigma;
+};
+EP_DEV void imp_field(const ImpTable& t, double rr2, double& vp, double& dl) {
+  const double rs = rsqrt(rr2);
+  double r = rr2 * rs;
+  r = fma(fma(-r, r, rr2), 0.5 * rs, r);
+  const double q = fma(r, t.rh, 1.5);
+  int i0 = (int)q;
+  // compared in FP32 and, for rr2 > 1.1e-6, by the exponent word (an FP64
+  // comparison is an FP64-pipe operation)
+  const float fr = (float)(q - (double)i0);
+  bool lo = fr < 0.5f;
+  const bool plain = __double2hiint(rr2) > 0x3eb27476 && fr > 1e-5f && fr < 1.0f - 1e-5f && fabsf(fr - 0.5f) > 1e-5f &&
+                     i0 < t.npot;
+  if (!plain) {
+    r = sqrt(rr2);
+    i0 = (int)(1.5 + r / t.h);
+    i0 = min(max(i0, 1), t.npot);
+    lo = r < (i0 - 1) * t.h;
+  }
+  const double2* c = reinterpret_cast<const double2*>(t.coef + ((lo ? 0 : t.npot + 2) + i0) * 8);
+  const double2 c0 = __ldg(c), c1 = __ldg(c + 1), c2 = __ldg(c + 2);
+  vp = r * (c0.x * r + c0.y) + c1.x;
+  dl = r * (c1.y * r + c2.x) + c2.y;
+  if (plain) dl *= rs * rs;
+  else dl = r > 1e-3 ? dl / rr2 : t.umax_sigma;
+}
+
+// A double as a field value.  The double-float split rounds to 24 bits in the
+// integer pipe (as (float)d rounds but for ties) and takes two FP64-pipe
+// operations, the difference and its conversion, where the converting
+// constructor takes four; values outside the FP32 range's middle use that.
+template <class T> EP_DEV T to_field(double d) { return (T)d; }
+template <> EP_DEV dfloat to_field<dfloat>(double d) {
+  const long long b = __double_as_longlong(d);
+  if ((b << 1) == 0) return dfloat(0.0f, 0.0f);
+  const unsigned e = (unsigned)(b >> 52) & 0x7ffu;
+  if (e - 923u > 226u) return dfloat(d);  // below 2^-100 or above 2^126, Inf, NaN
+  const long long rb = (b + 0x10000000ll) & ~0x1fffffffll;
+  const unsigned m = (unsigned)((rb & 0x7fffffffffffffffll) >> 29) - (896u << 23);
+  return dfloat(__uint_as_float(m | ((unsigned)(rb >> 32) & 0x80000000u)), (float)(d - __longlong_as_double(rb)));
+}
+
+// The field of the P-state impurity.  Bound by the FP64 pipe (about 45
+// operations a point with double-float stores, 35 in FP64; the table
+// arithmetic, a division by h and one by r^2 per point were 120): 96 x 160 x
+// 192 double-float 623 -> 292 us.
+template <class T>
+__global__ void __launch_bounds__(256) k_potenimp(Geo g, ColGrid cg, double xmax, double ymax, double zmax, double hx,
+                                                  double hy, double hz, double r0, double r1, double r2, ImpTable t,
+                                                  double2 iv0, double2 iv1, double2 iv2, double2 iv3, double2 iv4,
+                                                  double2 iv5, T* __restrict__ vpi, T* __restrict__ delta,
+                                                  T* __restrict__ uimp) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  double2* ys = reinterpret_cast<double2*>(smraw);  // y - r_imp,y of the chunk's rows and its square
+  const int y0 = blockIdx.y * cg.rows;
+  for (int i = threadIdx.x + 32 * threadIdx.y; i < cg.rows; i += 32 * blockDim.y) {
+    const double yy = coord(ymax, hy, y0 + i) - r1;
+    ys[i] = make_double2(yy, __dmul_rn(yy, yy));
+  }
+  __syncthreads();
+  double xx = 0, zz = 0, x2 = 0, z2 = 0, oxc = 0, oyc = 0, exc = 0, eyc = 0;
+  columns(
+      g, cg,
+      [&](int ix, int iz, long long) {
+        xx = coord(xmax, hx, ix) - r0;
+        zz = coord(zmax, hz, iz) - r2;
+        x2 = __dmul_rn(xx, xx);
+        z2 = __dmul_rn(zz, zz);
+        oxc = iv0.x * xx + iv4.x * zz;
+        oyc = iv0.y * xx + iv4.y * zz;
+        exc = iv1.x * xx + iv5.x * zz;
+        eyc = iv1.y * xx + iv5.y * zz;
+      },
+      [&](int iy, long long p) {
+        const double yy = ys[iy - y0].x;
+        const double rr2 = __dadd_rn(x2, __dadd_rn(ys[iy - y0].y, z2));  // rr2_nc's order
+        double vp, dl;
+        imp_field(t, rr2, vp, dl);
+        const double ox = iv2.x * yy + oxc, oy = iv2.y * yy + oyc, ex = iv3.x * yy + exc, ey = iv3.y * yy + eyc;
+        const double u = vp + dl * ((ox * ox + oy * oy) + (ex * ex + ey * ey));
+        vpi[p] = to_field<T>(vp);
+        delta[p] = to_field<T>(dl);
+        uimp[p] = to_field<T>(fmin(u, 1000.0));
+      },
+      [] {});
 }
 
 // D-state angular factors at x = r - rimp (potenimp.f90:68-117): the d
@@ -186,56 +289,127 @@ EP_DEV float interp_update_f(float r, int nint, float h, float rh, const float* 
   return f0 + d * (b + aa * d);
 }
 
-static __global__ void k_potenimp_f(Geo g, float xmax, float ymax, float zmax, float hx, float hy, float hz, float r0,
-                             float r1, float r2, const float* __restrict__ potpi, const float* __restrict__ potdel,
-                             int npot, float h, float rh, float umax_sigma, float2 iv0, float2 iv1, float2 iv2,
-                             float2 iv3, float2 iv4, float2 iv5, float* __restrict__ vpi, float* __restrict__ delta,
-                             float* __restrict__ uimp) {
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < g.N; p += (long long)gridDim.x * blockDim.x) {
-    int ix, iy, iz;
-    idx3(g, p, ix, iy, iz);
-    const float xx = ((float)ix * hx - xmax) - r0;
-    const float yy = ((float)iy * hy - ymax) - r1;
-    const float zz = ((float)iz * hz - zmax) - r2;
-    const float rr2 = xx * xx + (yy * yy + zz * zz);
-    const float r = sqrtf(rr2);
-    const float vp = interp_update_f(r, npot, h, rh, potpi);
-    const float dl = r > 1e-3f ? interp_update_f(r, npot, h, rh, potdel) / rr2 : umax_sigma;
-    const float ox = iv0.x * xx + iv2.x * yy + iv4.x * zz, oy = iv0.y * xx + iv2.y * yy + iv4.y * zz;
-    const float ex = iv1.x * xx + iv3.x * yy + iv5.x * zz, ey = iv1.y * xx + iv3.y * yy + iv5.y * zz;
-    const float u = vp + dl * ((ox * ox + oy * oy) + (ex * ex + ey * ey));
-    vpi[p] = vp;
-    delta[p] = dl;
-    uimp[p] = fminf(u, 1000.0f);
-  }
+// The coordinates from the impurity are FP64 differences rounded once, per
+// column and per row (in FP32 their rounding at the box's size, 2e-6 A, times
+// the slope of a cut-off core was 2e-5 of the field's maximum).
+static __global__ void __launch_bounds__(256)
+    k_potenimp_f(Geo g, ColGrid cg, double xmax, double ymax, double zmax, double hx, double hy, double hz, double r0,
+                 double r1, double r2, const float* __restrict__ potpi, const float* __restrict__ potdel, int npot,
+                 float h, float rh, float umax_sigma, float2 iv0, float2 iv1, float2 iv2, float2 iv3, float2 iv4,
+                 float2 iv5, float* __restrict__ vpi, float* __restrict__ delta, float* __restrict__ uimp) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  float* ys = reinterpret_cast<float*>(smraw);  // y - r_imp,y of the chunk's rows
+  const int y0 = blockIdx.y * cg.rows;
+  for (int i = threadIdx.x + 32 * threadIdx.y; i < cg.rows; i += 32 * blockDim.y)
+    ys[i] = (float)(coord(ymax, hy, y0 + i) - r1);
+  __syncthreads();
+  float xx = 0, zz = 0;
+  columns<4>(
+      g, cg,
+      [&](int ix, int iz, long long) {
+        xx = (float)(coord(xmax, hx, ix) - r0);
+        zz = (float)(coord(zmax, hz, iz) - r2);
+      },
+      [&](int iy, long long p) {
+        const float yy = ys[iy - y0];
+        const float rr2 = xx * xx + (yy * yy + zz * zz);
+        const float r = sqrtf(rr2);
+        const float vp = interp_update_f(r, npot, h, rh, potpi);
+        const float dl = r > 1e-3f ? interp_update_f(r, npot, h, rh, potdel) / rr2 : umax_sigma;
+        const float ox = iv0.x * xx + iv2.x * yy + iv4.x * zz, oy = iv0.y * xx + iv2.y * yy + iv4.y * zz;
+        const float ex = iv1.x * xx + iv3.x * yy + iv5.x * zz, ey = iv1.y * xx + iv3.y * yy + iv5.y * zz;
+        const float u = vp + dl * ((ox * ox + oy * oy) + (ex * ex + ey * ey));
+        vpi[p] = vp;
+        delta[p] = dl;
+        uimp[p] = fminf(u, 1000.0f);
+      },
+      [] {});
 }
 
-// FP32 engine, P state: forceimp sums and the six moments in compensated
-// FP32 per thread, FP64 across threads and blocks.
-static __global__ void k_impmoments_f(Geo g, const float* __restrict__ den, const float* __restrict__ dxd,
-                               const float* __restrict__ dyd, const float* __restrict__ dzd,
-                               const float* __restrict__ uimp, const float* __restrict__ vpi,
-                               const float* __restrict__ delta, float xmax, float ymax, float zmax, float hx, float hy,
-                               float hz, float r0, float r1, float r2, int izlo, int izhi,
-                               double* __restrict__ partials) {
-  Acc<float> acc[9];
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < g.N; p += (long long)gridDim.x * blockDim.x) {
-    int ix, iy, iz;
-    idx3(g, p, ix, iy, iz);
-    const float u = uimp[p];
-    acc[0].add(dxd[p] * u);
-    acc[1].add(dyd[p] * u);
-    if (iz >= izlo && iz < izhi) acc[2].add(dzd[p] * u);
-    const float xx = ((float)ix * hx - xmax) - r0, yy = ((float)iy * hy - ymax) - r1,
-                zz = ((float)iz * hz - zmax) - r2;
-    const float a1 = den[p], a2 = delta[p], a3 = vpi[p];
-    acc[3].add(a1 * (a2 * xx * xx + a3));
-    acc[4].add(a1 * a2 * xx * yy);
-    acc[5].add(a1 * a2 * xx * zz);
-    acc[6].add(a1 * (a2 * yy * yy + a3));
-    acc[7].add(a1 * a2 * yy * zz);
-    acc[8].add(a1 * (a2 * zz * zz + a3));
-  }
+// Exact or double-float products of field values for the sums: FP64 in FP64;
+// a pair of FP32 values (the product and its FMA error, 2^-47 of it at most)
+// for FP32 and double-float fields, whose sums are FP32 pairs (ep_reduce.cuh).
+EP_DEV double wmul(double a, double b) { return a * b; }
+EP_DEV dfloat wmul(dfloat a, dfloat b) { return a * b; }
+EP_DEV dfloat wmul(float a, float b) {
+  const float p = __fmul_rn(a, b);
+  return dfloat(p, __fmaf_rn(a, b, -p));
+}
+EP_DEV dfloat wmul(dfloat a, float b) {
+  const float p = __fmul_rn(a.hi, b);
+  return dd_fast2sum(p, __fmaf_rn(a.lo, b, __fmaf_rn(a.hi, b, -p)));
+}
+EP_DEV dfloat wmul(float a, dfloat b) { return wmul(b, a); }
+// The value of a per-thread sum in the arithmetic of its terms.
+EP_DEV double wvalue(const Neumaier<double>& a) { return a.s + a.c; }
+EP_DEV dfloat wvalue(const Kahan<dfloat>& a) { return dd_fast2sum(a.s, a.c); }
+EP_DEV float wvalue(const Kahan<float>& a) { return a.s - a.c; }
+EP_DEV float fmul1(float a, float b) { return a * b; }
+
+// P state: forceimp sums and the six moments (the matrix of the internal
+// variables).  Along a column only y varies, so a point adds four moments of
+// den Delta and den V_Pi (1, y, y^2) and the column's x and z factors are
+// applied once per column: seven products and seven compensated sums a point
+// in the fields' own arithmetic (FP32; pairs of FP32 values in double-float;
+// FP64).  In double-float the products' 2^-45 is below the fields' own
+// rounding, and the FP64 conversions, products and sums of the one-point form
+// (about 120 operations a point on the FP64 pipe) go: 96 x 160 x 192 896 ->
+// 46 us; FP64 64 x 64 x 80 360 -> 123 us; FP32 256 x 256 x 320
+// 168 -> 120 us (memory: seven fields read).
+template <class T>
+__global__ void __launch_bounds__(256) k_impmoments(Geo g, ColGrid cg, const T* __restrict__ den,
+                                                    const T* __restrict__ dxd, const T* __restrict__ dyd,
+                                                    const T* __restrict__ dzd, const T* __restrict__ uimp,
+                                                    const T* __restrict__ vpi, const T* __restrict__ delta,
+                                                    double xmax, double ymax, double zmax, double hx, double hy,
+                                                    double hz, double r0, double r1, double r2, int izlo, int izhi,
+                                                    double* __restrict__ partials) {
+  constexpr bool F = std::is_same<T, float>::value;
+  auto mul = [](T a, T b) {
+    if constexpr (F) return fmul1(a, b);
+    else return wmul(a, b);
+  };
+  extern __shared__ __align__(16) unsigned char smraw[];
+  T* ys = reinterpret_cast<T*>(smraw);  // y - r_imp,y of the chunk's rows
+  const int y0 = blockIdx.y * cg.rows;
+  for (int i = threadIdx.x + 32 * threadIdx.y; i < cg.rows; i += 32 * blockDim.y)
+    ys[i] = T(coord(ymax, hy, y0 + i) - r1);
+  __syncthreads();
+  Acc<T> acc[9];
+  Acc<T> sv, s0, s1, s2;  // along the column: den V_Pi and den Delta (1, y, y^2)
+  T xx = T(0), zz = T(0);
+  bool fz = false;
+  columns<F ? 4 : 2>(
+      g, cg,
+      [&](int ix, int iz, long long) {
+        xx = T(coord(xmax, hx, ix) - r0);
+        zz = T(coord(zmax, hz, iz) - r2);
+        fz = iz >= izlo && iz < izhi;
+        sv = s0 = s1 = s2 = Acc<T>();
+      },
+      [&](int iy, long long p) {
+        const T u = uimp[p], a1 = den[p], yy = ys[iy - y0];
+        acc[0].add(mul(dxd[p], u));
+        acc[1].add(mul(dyd[p], u));
+        if (fz) acc[2].add(mul(dzd[p], u));
+        const T d = mul(a1, delta[p]), dy = mul(d, yy);
+        sv.add(mul(a1, vpi[p]));
+        s0.add(d);
+        s1.add(dy);
+        s2.add(mul(dy, yy));
+      },
+      [&] {
+        const T V = wvalue(sv), D = wvalue(s0), Dx = mul(xx, D), Dz = mul(zz, D), Dy = wvalue(s1);
+        acc[3].add(V);
+        acc[3].add(mul(xx, Dx));
+        acc[4].add(mul(xx, Dy));
+        acc[5].add(mul(xx, Dz));
+        acc[6].add(V);
+        acc[6].add(wvalue(s2));
+        acc[7].add(mul(zz, Dy));
+        acc[8].add(V);
+        acc[8].add(mul(zz, Dz));
+      });
   block_reduce_store_acc<9>(acc, partials);
 }
 
@@ -250,85 +424,187 @@ __global__ void k_normsum(const C2<T>* __restrict__ psi, long long N, double* __
   block_reduce_store_acc<1>(acc, partials);
 }
 
-// Complex first derivative from global memory.
-template <class T>
-EP_DEV C2<T> d1c_global(const C2<T>* __restrict__ f, long long p, int i, int n, long long st, const T* w, int R,
-                        int periodic) {
-  C2<T> s = cmk<T>(T(0), T(0));
-  for (int k = 1; k <= R; ++k) {
-    int ip = i + k, im = i - k;
-    C2<T> fp, fm;
-    if (ip >= n) fp = periodic ? f[p + (long long)(ip - n - i) * st] : cmk<T>(T(0), T(0));
-    else fp = f[p + (long long)k * st];
-    if (im < 0) fm = periodic ? f[p + (long long)(im + n - i) * st] : cmk<T>(T(0), T(0));
-    else fm = f[p - (long long)k * st];
-    s = s + w[k] * (fp - fm);
+// Running sum of w_k (a_k - b_k) of complex values: paired FMAs, or the
+// unnormalised double-float accumulation of ep_dd.cuh.
+template <class T> struct DiffSum {
+  C2<T> s;
+  EP_DEV DiffSum() : s(cmk<T>(T(0), T(0))) {}
+  EP_DEV void add(T w, C2<T> a, C2<T> b) { s = vfma(w, vsub(a, b), s); }
+  EP_DEV C2<T> value() const { return s; }
+};
+#if defined(__CUDA_ARCH__)
+template <> struct DiffSum<dfloat> {
+  dd2_acc s;
+  EP_DEV DiffSum() : s{make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)} {}
+  EP_DEV void add(dfloat w, dfloat2 a, dfloat2 b) {
+    float2 ph, pl;
+    dd2_wdiff(w, a, b, ph, pl);
+    dd2_add(s, ph, pl);
   }
-  return s;
-}
+  EP_DEV dfloat2 value() const { return dd2_value(s); }
+};
+#endif
 
-template <class T>
-__global__ void k_energy(Geo g, FdW<T> fd, Phys ph, const C2<T>* __restrict__ psi, const T* __restrict__ den,
-                         const T* __restrict__ dencg, const T* __restrict__ delj4, const T* __restrict__ falfs,
-                         const T* __restrict__ dxd, const T* __restrict__ dyd, const T* __restrict__ dzd,
-                         const T* __restrict__ ix_, const T* __restrict__ iy_, const T* __restrict__ iz_,
-                         const T* __restrict__ uimp, double xmax, double ymax, double zmax, double hx, double hy,
-                         double hz, double r0, double r1, double r2, double zexc, const __grid_constant__ PotDev vplus,
-                         int impurity, double* __restrict__ partials) {
-  Acc<double> acc[8];
-  const bool otc = ph.core == 1;
-  const double aux1 = 0.5 * ph.cp4, aux2 = (1.0 / 3.0) * ph.cpp4;
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < g.N; p += (long long)gridDim.x * blockDim.x) {
-    int ix, iy, iz;
-    idx3(g, p, ix, iy, iz);
-    const C2<T> dx = d1c_global(psi, p, ix, g.nx, 1, fd.w1[0], fd.R, fd.periodic);
-    const C2<T> dy = d1c_global(psi, p, iy, g.ny, (long long)g.nx, fd.w1[1], fd.R, fd.periodic);
-    const C2<T> dz = d1c_global(psi, p, iz, g.nz, (long long)g.nx * g.ny, fd.w1[2], fd.R, fd.periodic);
-    const double dn = dbl(den[p]), cg = dbl(dencg[p]);
-    acc[0].add((dbl(dx.x) * dbl(dx.x) + dbl(dx.y) * dbl(dx.y)) + (dbl(dy.x) * dbl(dy.x) + dbl(dy.y) * dbl(dy.y)) +
-               (dbl(dz.x) * dbl(dz.x) + dbl(dz.y) * dbl(dz.y)));
-    acc[1].add((double)delj4[p] * dn);
-    acc[2].add(dn * (cg * cg) * (aux1 + aux2 * cg));
-    if (otc)
-      acc[3].add(dbl(falfs[p]) * (dbl(dxd[p]) * dbl(ix_[p]) + dbl(dyd[p]) * dbl(iy_[p]) + dbl(dzd[p]) * dbl(iz_[p])));
-    acc[4].add(dn * (1.0 + tanh(ph.beta * (dn - ph.den_m))));
-    if (impurity) {
-      const double a = r0 - coord(xmax, hx, ix), b = r1 - coord(ymax, hy, iy), c = r2 - coord(zmax, hz, iz);
-      const double r = sqrt(__dadd_rn(__dadd_rn(__dmul_rn(a, a), __dmul_rn(b, b)), __dmul_rn(c, c)));
-      if (r >= zexc) {
-        acc[5].add(dn * (double)uimp[p]);
-        acc[6].add(dn * pot_eval(vplus, r));
-      }
+// Complex first derivative at c along an axis of n points with element stride
+// st (index i), from global memory.  LANE: the index differs across the warp
+// (x), so each neighbour wraps by a selection; else (y, z) whole warps are
+// inside and step two pointers.
+template <class T, bool LANE>
+EP_DEV C2<T> d1c_global(const C2<T>* __restrict__ c, int i, int n, long long st, const T* w, int R, int periodic) {
+  DiffSum<T> s;
+  const C2<T> zero = cmk<T>(T(0), T(0));
+  if (!LANE && i >= R && i < n - R) {
+    const C2<T>*u = c + st, *d = c - st;
+    for (int k = 1; k <= R; ++k, u += st, d -= st) s.add(w[k], __ldg(u), __ldg(d));
+  } else {
+    for (int k = 1; k <= R; ++k) {
+      const bool ou = i + k >= n, od = i - k < 0;
+      const long long u = ou ? k - n : k, d = od ? n - k : -k;
+      s.add(w[k], ou && !periodic ? zero : __ldg(c + u * st), od && !periodic ? zero : __ldg(c + d * st));
     }
-    acc[7].add(dn);
   }
-  block_reduce_store_acc<8>(acc, partials);
+  return s.value();
 }
 
-template <class T>
-__global__ void k_impmoments(Geo g, const T* __restrict__ den, const T* __restrict__ dxd,
-                             const T* __restrict__ dyd, const T* __restrict__ dzd, const T* __restrict__ uimp,
-                             const T* __restrict__ vpi, const T* __restrict__ delta, double xmax, double ymax,
-                             double zmax, double hx, double hy, double hz, double r0, double r1, double r2,
-                             int izlo, int izhi, double* __restrict__ partials) {
-  Acc<double> acc[9];
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < g.N; p += (long long)gridDim.x * blockDim.x) {
-    int ix, iy, iz;
-    idx3(g, p, ix, iy, iz);
-    const double u = dbl(uimp[p]);
-    acc[0].add((double)dxd[p] * u);
-    acc[1].add((double)dyd[p] * u);
-    if (iz >= izlo && iz < izhi) acc[2].add((double)dzd[p] * u);
-    const double xx = coord(xmax, hx, ix) - r0, yy = coord(ymax, hy, iy) - r1, zz = coord(zmax, hz, iz) - r2;
-    const double a1 = dbl(den[p]), a2 = dbl(delta[p]), a3 = dbl(vpi[p]);
-    acc[3].add(a1 * (a2 * xx * xx + a3));
-    acc[4].add(a1 * a2 * xx * yy);
-    acc[5].add(a1 * a2 * xx * zz);
-    acc[6].add(a1 * (a2 * yy * yy + a3));
-    acc[7].add(a1 * a2 * yy * zz);
-    acc[8].add(a1 * (a2 * zz * zz + a3));
+// 1 + tanh(beta (den - den_m)) of the solid penalty.  For 2 beta (den - den_m)
+// < -25 (a liquid's density: -28) it is 2 e / (1 + e), e = exp(2 beta (den -
+// den_m)) < 1.4e-11, from the FP32 exponential: its error, below 3e-6 e, is
+// under the 1.1e-16 that the cancellation in FP64's 1 + tanh leaves there.
+EP_DEV double one_plus_tanh(const Phys& ph, double dn) {
+  const float y = (float)(2.0 * ph.beta * (dn - ph.den_m));
+  if (y < -25.0f) {
+    const float e = expf(y);
+    return (double)(2.0f * e);
   }
-  block_reduce_store_acc<9>(acc, partials);
+  return 1.0 + tanh(ph.beta * (dn - ph.den_m));
+}
+template <class T>
+EP_DEV dfloat one_plus_tanh_f(const Phys& ph, T dn) {
+  const float b2 = 2.0f * ph.f.beta, y = fmaf(b2, (float)dn, -b2 * ph.f.den_m);
+  if (y < -25.0f) return dfloat(2.0f * expf(y));
+  return dfloat(1.0 + tanh(ph.beta * (dbl(dn) - ph.den_m)));
+}
+
+// Energy integrals.  W: the arithmetic of the terms (W = double: FP64; W =
+// dfloat: pairs of FP32 values, exact products of FP32 fields, 2^-45 for
+// double-float ones, summed in FP32 pairs).  The FP64 form of every engine was
+// bound by the FP64 pipe (about 380 operations a point: conversions, tanh,
+// eight Neumaier sums); FP32 fields in pairs leave the pipe to a U+ that
+// is no Morse potential (its distance and pair potential).  128^3, impurity with a Morse U+: FP32 1142 ->
+// 169 us, double-float 1333 -> 272, FP64 1260 -> 953 (64^3: 426
+// -> 151).  The caller falls back to W = double where the pairs' FP32
+// range does not hold the sums.
+template <class T, class W>
+__global__ void __launch_bounds__(256) k_energy(Geo g, ColGrid cg, const __grid_constant__ FdW<T> fd, Phys ph, const C2<T>* __restrict__ psi,
+                                                const T* __restrict__ den, const T* __restrict__ dencg,
+                                                const T* __restrict__ delj4, const T* __restrict__ falfs,
+                                                const T* __restrict__ dxd, const T* __restrict__ dyd,
+                                                const T* __restrict__ dzd, const T* __restrict__ ix_,
+                                                const T* __restrict__ iy_, const T* __restrict__ iz_,
+                                                const T* __restrict__ uimp, double xmax, double ymax, double zmax,
+                                                double hx, double hy, double hz, double r0, double r1, double r2,
+                                                double zexc, const __grid_constant__ PotDev vplus, int impurity,
+                                                double* __restrict__ partials) {
+  constexpr bool D64 = std::is_same<W, double>::value;
+  Acc<W> acc[8];
+  const bool otc = ph.core == 1;
+  // FP32 fields: a Morse U+ in pairs of FP32 values (2^-36 and better; in FP64
+  // its root and exponential were 200 us of the 255 at 128^3)
+  const bool pair_u = std::is_same<T, float>::value && !D64 && vplus.kind == EP_POT_MORSE && zexc <= 0.0;
+  // r in FP64 is needed for the exclusion radius and any other U+ that is not
+  // zero everywhere
+  const bool need_r = impurity && !pair_u && (vplus.kind != EP_POT_NULL || !(zexc <= 0.0));
+  extern __shared__ __align__(16) unsigned char smraw[];
+  dfloat* ys = reinterpret_cast<dfloat*>(smraw);  // r_imp,y - y of the chunk's rows (pair_u)
+  const int y0 = blockIdx.y * cg.rows;
+  dfloat ac(0.0f, 0.0f), De = ac, re = ac, al = ac;
+  if (pair_u) {
+    De = dfloat(vplus.par[0]);
+    re = dfloat(vplus.par[1]);
+    al = dfloat(vplus.par[2]);
+    for (int i = threadIdx.x + 32 * threadIdx.y; i < cg.rows; i += 32 * blockDim.y)
+      ys[i] = dfloat(r1 - coord(ymax, hy, y0 + i));
+    __syncthreads();
+  }
+  int ix = 0, iz = 0;
+  double a2 = 0, c2 = 0;
+  const long long sz = (long long)g.nx * g.ny;
+  columns(
+      g, cg,
+      [&](int i, int k, long long) {
+        ix = i;
+        iz = k;
+        if (need_r) {
+          const double a = r0 - coord(xmax, hx, ix), c = r2 - coord(zmax, hz, iz);
+          a2 = __dmul_rn(a, a);
+          c2 = __dmul_rn(c, c);
+        } else if (pair_u) {
+          const double a = r0 - coord(xmax, hx, ix), c = r2 - coord(zmax, hz, iz);
+          ac = dfloat(a * a + c * c);
+        }
+      },
+      [&](int iy, long long p) {
+        const C2<T> dx = d1c_global<T, true>(psi + p, ix, g.nx, 1, fd.w1[0], fd.R, fd.periodic);
+        const C2<T> dy = d1c_global<T, false>(psi + p, iy, g.ny, (long long)g.nx, fd.w1[1], fd.R, fd.periodic);
+        const C2<T> dz = d1c_global<T, false>(psi + p, iz, g.nz, sz, fd.w1[2], fd.R, fd.periodic);
+        const T dn = den[p], cg_ = dencg[p], lj = delj4[p];
+        bool inside = impurity != 0;
+        double r = 0.0;
+        if (need_r) {
+          const double b = r1 - coord(ymax, hy, iy);
+          r = sqrt(__dadd_rn(__dadd_rn(a2, __dmul_rn(b, b)), c2));
+          inside = inside && r >= zexc;
+        }
+        if constexpr (D64) {
+          const double n = dbl(dn), c = dbl(cg_);
+          acc[0].add((dbl(dx.x) * dbl(dx.x) + dbl(dx.y) * dbl(dx.y)) +
+                     (dbl(dy.x) * dbl(dy.x) + dbl(dy.y) * dbl(dy.y)) +
+                     (dbl(dz.x) * dbl(dz.x) + dbl(dz.y) * dbl(dz.y)));
+          acc[1].add(dbl(lj) * n);
+          acc[2].add(n * (c * c) * (0.5 * ph.cp4 + (1.0 / 3.0) * ph.cpp4 * c));
+          if (otc)
+            acc[3].add(dbl(falfs[p]) *
+                       (dbl(dxd[p]) * dbl(ix_[p]) + dbl(dyd[p]) * dbl(iy_[p]) + dbl(dzd[p]) * dbl(iz_[p])));
+          acc[4].add(n * one_plus_tanh(ph, n));
+          if (inside) {
+            acc[5].add(n * dbl(uimp[p]));
+            if (vplus.kind != EP_POT_NULL) acc[6].add(n * pot_eval(vplus, r));
+          }
+          acc[7].add(n);
+        } else {
+          acc[0].add(wmul(dx.x, dx.x));
+          acc[0].add(wmul(dx.y, dx.y));
+          acc[0].add(wmul(dy.x, dy.x));
+          acc[0].add(wmul(dy.y, dy.y));
+          acc[0].add(wmul(dz.x, dz.x));
+          acc[0].add(wmul(dz.y, dz.y));
+          acc[1].add(wmul(lj, dn));
+          acc[2].add(wmul(wmul(wmul(cg_, cg_), dn), ph.d.a0 + wmul(ph.d.a1, cg_)));
+          if (otc)
+            acc[3].add(wmul((wmul(dxd[p], ix_[p]) + wmul(dyd[p], iy_[p])) + wmul(dzd[p], iz_[p]), falfs[p]));
+          acc[4].add(wmul(one_plus_tanh_f(ph, dn), dn));
+          if (inside) {
+            acc[5].add(wmul(dn, uimp[p]));
+            if (pair_u) {
+              const dfloat b = ys[iy - y0], rd = sqrt(ac + b * b);
+              const float rc = (float)vplus.r_cutoff;
+              dfloat V;
+              if (rc > 0.0f && fabsf(rd.hi - rc) <= 1e-5f * rc) V = dfloat(pot_eval(vplus, (double)rd));
+              else if (rd.hi < rc) V = dfloat(vplus.umax);
+              else {
+                const dfloat e = dd_exp(-(al * (rd - re)));
+                V = De * (e * e - dfloat(2.0f, 0.0f) * e);
+              }
+              acc[6].add(wmul(V, dn));
+            } else if (vplus.kind != EP_POT_NULL) {
+              acc[6].add(wmul(dfloat(pot_eval(vplus, r)), dn));
+            }
+          }
+          acc[7].add(dfloat(dn));
+        }
+      },
+      [] {});
+  block_reduce_store_acc<8>(acc, partials);
 }
 
 // ---------------------------------------------------------------------------

@@ -100,30 +100,56 @@ EP_DEV void warp_pair_sum(F& s, F& c) {
   }
 }
 
-// Warp 0 finishes the per-warp pairs red_s/red_c[q][warp] of a block and
-// stores the block's pair of every q in QMASK.
-template <int NQ, unsigned QMASK, class F>
-EP_DEV void block_pairs_store(F (&red_s)[NQ][32], F (&red_c)[NQ][32], int lane, int warp, int nw,
-                              double* __restrict__ partials) {
-  if (warp == 0) {
-    const long long nb = (long long)gridDim.x * gridDim.y * gridDim.z;
-    const long long b = blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
+// Warp sums of N pairs at once (N a power of two, at most 32): while more
+// than one sum is left, the lanes of one half of the exchange keep one half of
+// the sums and hand the other half over, so that a step adds as many pairs as
+// it leaves (9 pair additions for 8 sums, 16 for 16, where one tree per sum
+// takes 40 and 80: the FP64 pipe needs 16 cycles for a warp instruction).
+// Sum multi_index<N>(lane) ends in s[0], c[0] of every lane.
+template <int N, int O = 16, class F>
+EP_DEV void warp_multi_sum(F* s, F* c) {
+  static_assert(N >= 1 && N <= 32 && (N & (N - 1)) == 0, "a power of two of sums");
+  if constexpr (O > 0) {
+    if constexpr (N > 1) {
+      const bool up = (threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z)) & O;
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-      if (!((QMASK >> q) & 1u)) continue;
-      F s = lane < nw ? red_s[q][lane] : F(0), c = lane < nw ? red_c[q][lane] : F(0);
-      warp_pair_sum(s, c);
-      if (lane == 0) {
-        // the pair widened to FP64 exactly (an FP32 pair gives its two
-        // values; TwoSum of them is exact in FP64)
-        double hs, he;
-        two_sum((double)s, (double)c, hs, he);
-        partials[b * NQ + q] = hs;
-        partials[nb * NQ + b * NQ + q] = he;
+      for (int i = 0; i < N / 2; ++i) {
+        const F gs = up ? s[i] : s[i + N / 2], gc = up ? c[i] : c[i + N / 2];
+        F ks = up ? s[i + N / 2] : s[i], kc = up ? c[i + N / 2] : c[i];
+        pair_add(ks, kc, __shfl_xor_sync(0xffffffffu, gs, O), __shfl_xor_sync(0xffffffffu, gc, O));
+        s[i] = ks;
+        c[i] = kc;
       }
+      warp_multi_sum<N / 2, O / 2>(s, c);
+    } else {
+      pair_add(s[0], c[0], __shfl_xor_sync(0xffffffffu, s[0], O), __shfl_xor_sync(0xffffffffu, c[0], O));
+      warp_multi_sum<1, O / 2>(s, c);
     }
   }
 }
+template <int N>
+EP_DEV int multi_index(int lane) {
+  int q = 0;
+#pragma unroll
+  for (int n = N / 2, o = 16; n > 0; n /= 2, o /= 2) q += (lane & o) ? n : 0;
+  return q;
+}
+
+// The sums of QMASK among NQ: how many, the k-th of them, and their count
+// rounded up to a power of two.
+template <int NQ, unsigned QMASK> struct QSel {
+  static constexpr unsigned M = NQ >= 32 ? QMASK : QMASK & ((1u << NQ) - 1u);
+  EP_HD static constexpr int count(unsigned m) { return m ? 1 + count(m & (m - 1)) : 0; }
+  EP_HD static constexpr int kth(int k) {
+    for (int q = 0; q < NQ; ++q)
+      if ((M >> q) & 1u)
+        if (k-- == 0) return q;
+    return -1;
+  }
+  static constexpr int N = count(M);
+  EP_HD static constexpr int pad(int n) { return n <= 1 ? 1 : 2 * pad((n + 1) / 2); }
+  static constexpr int NP = pad(N);
+};
 
 // Block reduction of per-thread accumulators into the block's pairs, for
 // the sums q whose bit is set in QMASK (the others are not stored).  FP32
@@ -133,28 +159,53 @@ EP_DEV void block_pairs_store(F (&red_s)[NQ][32], F (&red_c)[NQ][32], int lane, 
 template <int NQ, unsigned QMASK = ~0u, class A>
 EP_DEV void block_reduce_store_acc(A (&acc)[NQ], double* __restrict__ partials) {
   typedef typename A::value_type T;
-  __shared__ T red_s[NQ][32], red_c[NQ][32];
+  typedef QSel<NQ, QMASK> Q;
+  __shared__ T red_s[Q::NP][32], red_c[Q::NP][32];
   const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
   const int nth = blockDim.x * blockDim.y * blockDim.z;
   const int lane = tid & 31, warp = tid >> 5, nw = (nth + 31) >> 5;
+  const int mine = multi_index<Q::NP>(lane);
+  const bool first = (lane & (32 / Q::NP - 1)) == 0;  // one lane per sum
+  T s[Q::NP], c[Q::NP];
 #pragma unroll
-  for (int q = 0; q < NQ; ++q) {
-    if (!((QMASK >> q) & 1u)) continue;
-    T s = acc[q].s, c = acc[q].lo();
-    warp_pair_sum(s, c);
-    if (lane == 0) {
-      red_s[q][warp] = s;
-      red_c[q][warp] = c;
-    }
+  for (int k = 0; k < Q::NP; ++k) {
+    s[k] = k < Q::N ? acc[k < Q::N ? Q::kth(k) : 0].s : T(0);
+    c[k] = k < Q::N ? acc[k < Q::N ? Q::kth(k) : 0].lo() : T(0);
+  }
+  warp_multi_sum<Q::NP>(s, c);
+  if (first) {
+    red_s[mine][warp] = s[0];
+    red_c[mine][warp] = c[0];
   }
   __syncthreads();
-  block_pairs_store<NQ, QMASK>(red_s, red_c, lane, warp, nw, partials);
+  if (warp == 0) {
+#pragma unroll
+    for (int k = 0; k < Q::NP; ++k) {
+      s[k] = lane < nw ? red_s[k][lane] : T(0);
+      c[k] = lane < nw ? red_c[k][lane] : T(0);
+    }
+    warp_multi_sum<Q::NP>(s, c);
+    if (first && mine < Q::N) {
+      int q = 0;
+#pragma unroll
+      for (int k = 0; k < Q::N; ++k)
+        if (k == mine) q = Q::kth(k);
+      const long long nb = (long long)gridDim.x * gridDim.y * gridDim.z;
+      const long long b = blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
+      // the pair widened to FP64 exactly (an FP32 pair gives its two values;
+      // TwoSum of them is exact in FP64)
+      double hs, he;
+      two_sum((double)s[0], (double)c[0], hs, he);
+      partials[b * NQ + q] = hs;
+      partials[nb * NQ + b * NQ + q] = he;
+    }
+  }
 }
 
 // Sum of the block pairs of a reduction -> sc->sums[out0 + q] for the q in
 // qmask: warp w takes q = w, w + nwarps, ... (Neumaier over each lane's
 // blocks, then a pair tree across the warp).  mode 1: corrector epilogue
-// (norm, mu, renormalisation factor), mode 2: norm only.
+// (norm, mu, renormalisation factor).
 EP_DEV void finalize_block(const double* partials, int nblocks, int nq, DevScalars* sc, int out0, int mode,
                            double N, double dxyz, double n4, int renorm, int stats = 1, unsigned qmask = ~0u) {
   const int tid = threadIdx.x + blockDim.x * threadIdx.y;
@@ -186,11 +237,6 @@ EP_DEV void finalize_block(const double* partials, int nblocks, int nq, DevScala
         sc->errHe = sc->sums[out0] / N;
       }
       sc->scale = (renorm && norm > 0.0) ? sqrt(n4 / norm) : 1.0;
-    } else if (mode == 2) {
-      const double norm = sc->sums[out0] * dxyz;
-      sc->norm = norm;
-      sc->scale = norm > 0.0 ? sqrt(n4 / norm) : 1.0;
-      bad |= !(norm > 0.0);
     }
     if (bad) atomicOr(&sc->flags, (unsigned)EP_FLAG_NONFINITE);
   }
