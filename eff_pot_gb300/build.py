@@ -15,6 +15,9 @@ DRIVER_SRC = ["ep_fortran_io.cpp", "ep_dft4he3d.cpp"]
 UNITS = ["ep_engine_fp64.cu", "ep_engine_fp32.cu", "ep_engine_dd.cu", "ep_engine_dd_x.cu", "ep_engine_dd_xk0.cu",
          "ep_engine_dd_fft.cu", "ep_engine_dd_march.cu", "ep_common.cu", "ep_api.cu", "ep_noalloc.cu",
          "ep_select_pot.cu"] + [f"ep_yz_{t}_{p}.cu" for t in ("dd", "fp64", "fp32") for p in "dcba"]
+UNITS += [f"ep_xw_{t}_{p}.cu" for t in ("dd", "fp64", "fp32") for p in "dcba"]
+# the slowest units first
+UNITS.sort(key=lambda u: ("_dd" not in u, "engine" in u))
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
          "-I" + os.path.join(ROOT, "include")]

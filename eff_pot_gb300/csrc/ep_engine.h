@@ -159,8 +159,8 @@ class Engine {
   int x_attrs();
   int fft_attrs();
   int x_pass(int which, bool otc);
-  template <int N2> int x_launch(int which, bool otc);
-  template <int N2> int x_attrs_n2();
+  int x_launch(int which, bool otc);  // the general engine's X passes
+  int x_attrs_general();
   int march_setup();
   long long bytes = 0;
   Phys phys{};

@@ -8,6 +8,7 @@
 #include "ep_dstate.h"
 #include "ep_engine.h"
 #include "ep_kernels_impl.cuh"
+#include "ep_xw.cuh"
 #include "ep_yz.cuh"
 
 #define EP_RED_BLOCKS 1216
@@ -1314,7 +1315,7 @@ int Engine<T>::autotune(std::string* report) {
     const int xreal[4] = {0, 4, 4, 1};
     for (int round = 0; round < 2; ++round) {
       for (int cls = 0; cls < 6; ++cls) {
-        if ((cls == 4 && yz_kernels<T>(g.ny)) || (cls == 5 && yz_kernels<T>(g.nz))) continue;
+        if ((cls < 4 && xw_kernels<T>(g.nx / 2)) || (cls == 4 && yz_kernels<T>(g.ny)) || (cls == 5 && yz_kernels<T>(g.nz))) continue;
         const Shapes keep = shp;
         Shapes bestS = shp;
         float best = cur;
@@ -1366,70 +1367,77 @@ done:
 #if EP_ENGINE_PARTS & EP_PART_X
 template <class T>
 int Engine<T>::x_attrs() {
-  int r;
-  if ((r = x_attrs_n2<0>())) return r;
-  if constexpr (std::is_same<T, dfloat>::value) return EP_OK;  // general engine only
-  if ((r = x_attrs_n2<16>()) || (r = x_attrs_n2<32>()) || (r = x_attrs_n2<64>()) || (r = x_attrs_n2<128>()))
-    return r;
-  if constexpr (sizeof(T) == 4) {
-    if ((r = x_attrs_n2<48>()) || (r = x_attrs_n2<80>()) || (r = x_attrs_n2<96>())) return r;
+  if (const XWKernels* k = xw_kernels<T>(g.nx / 2)) {
+    for (int i = 0; i < 4; ++i)
+      cudaFuncSetAttribute(k->x[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k->smem[i]);
+    return EP_OK;
   }
-  return EP_OK;
+  return x_attrs_general();
 }
 
-// X pass `which` (1..4) of poten on the register transform of this grid's
-// half-lines (N2 = 0: the general engine).
+// X pass `which` (1..4) of poten: the kernels of this grid's half-line length,
+// or the general engine.
 template <class T>
 int Engine<T>::x_pass(int which, bool otc) {
-  if constexpr (std::is_same<T, dfloat>::value) return x_launch<0>(which, otc);
-  switch (x_reg_n2<T>(g.nx / 2)) {
-    case 16: return x_launch<16>(which, otc);
-    case 32: return x_launch<32>(which, otc);
-    case 64: return x_launch<64>(which, otc);
-    case 128: return x_launch<128>(which, otc);
-    case 48: if constexpr (sizeof(T) == 4) return x_launch<48>(which, otc); break;
-    case 80: if constexpr (sizeof(T) == 4) return x_launch<80>(which, otc); break;
-    case 96: if constexpr (sizeof(T) == 4) return x_launch<96>(which, otc); break;
-    default: break;
+  const XWKernels* k = xw_kernels<T>(g.nx / 2);
+  if (!k) return x_launch(which, otc);
+  static const char* const names[4] = {"x1_r2c_den", "x2_c2r_r2c", "x3_c2r_r2c", "x4_c2r_ualpha"};
+  long long nlines = (long long)g.ny * g.nz;
+  XWArgs<T> a{};
+  for (int i = 0; i < 4; ++i) {
+    a.in[i] = Tb[i];
+    a.out[i] = S[i];
   }
-  return x_launch<0>(which, otc);
+  a.den = den; a.dxd = dxd; a.dyd = dyd; a.dzd = dzd;
+  a.dencg = dencg; a.delj4 = delj4; a.pot4 = pot4; a.falfs = falfs;
+  a.intx = intx; a.inty = inty; a.intz = intz; a.gy = gy; a.gz = gz; a.dgx = dgx; a.ualphas = ualphas;
+  a.dyz = dyz;
+  a.twx = twx;
+  a.keep = 1;
+  void* args[] = {&nlines, &phys, &fd, &a};
+  cudaEvent_t ev = nullptr;
+  int c = -1;
+  prof->begin(st, names[which - 1], ev, c);
+  cudaError_t e = cudaLaunchKernel(k->x[which - 1], dim3((unsigned)((nlines + k->lines - 1) / k->lines)),
+                                   dim3(k->threads), args, k->smem[which - 1], st);
+  prof->end(st, c, ev);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  return cuda_ok(e, names[which - 1]);
 }
 #endif
 
 #if EP_ENGINE_PARTS & EP_PART_XK
 template <class T>
-template <int N2>
-int Engine<T>::x_attrs_n2() {
+int Engine<T>::x_attrs_general() {
   const int big = 220 * 1024;
-  cudaFuncSetAttribute(k_x1<T, N2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(k_x2<T, N2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(k_x3<T, N2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(k_x4<T, N2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(k_x1<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(k_x2<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(k_x3<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(k_x4<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   return EP_OK;
 }
 
 template <class T>
-template <int N2>
 int Engine<T>::x_launch(int which, bool otc) {
   const long long nlines = (long long)g.ny * g.nz;
   if (which == 1) {
     const int nl = x_lines(0, 0);
-    auto k = k_x1<T, N2>;
+    auto k = k_x1<T>;
     EP_LAUNCH("x1_r2c_den", k, (unsigned)((nlines + nl - 1) / nl), shp.xthr[0], x_smem(nl, 0), g, den, S[0], p2, twx, nl);
   } else if (which == 2) {
     const int nl = x_lines(1, otc ? 3 : 2);
-    auto k = k_x2<T, N2>;
+    auto k = k_x2<T>;
     EP_LAUNCH("x2_c2r_r2c", k, (unsigned)((nlines + nl - 1) / nl), shp.xthr[1], x_smem(nl, otc ? 3 : 2), g, phys, Tb[0],
               Tb[1], Tb[2], den, dxd, dyd, dzd, dencg, delj4, pot4, falfs, S[0], S[1], S[2], S[3], p2, twx, nl);
   } else if (which == 3) {
     const int nl = x_lines(2, otc ? 4 : 1);
-    auto k = k_x3<T, N2>;
+    auto k = k_x3<T>;
     EP_LAUNCH("x3_c2r_r2c", k, (unsigned)((nlines + nl - 1) / nl), shp.xthr[2], x_smem(nl, otc ? 4 : 1), g, phys, fd,
               Tb[0], Tb[1], Tb[2], Tb[3], den, dxd, dyd, dzd, falfs, pot4, intx, inty, intz, gy, gz, dgx, S[0], p2, twx,
               nl);
   } else {
     const int nl = x_lines(3, 1);
-    auto k = k_x4<T, N2>;
+    auto k = k_x4<T>;
     EP_LAUNCH("x4_c2r_ualpha", k, (unsigned)((nlines + nl - 1) / nl), shp.xthr[3], x_smem(nl, 1), g, phys, Tb[0], den,
               dgx, dyz, pot4, ualphas, p2, twx, nl);
   }

@@ -142,8 +142,15 @@ template <class T> struct Pen {
     den_m = k.den_m;
   }
 };
+// FP64: where 2 beta (den - den_m) < -26 (e = exp of it < 5.2e-12; a liquid's
+// density gives -28) the penalty is C e (2 + 4 beta den), from the FP32
+// exponential: its error, below 1e-6 of that, is under the rounding of FP64's
+// 1 + tanh there (1.1e-16 C), and tanh was most of X4's FP64 work.
 EP_DEV double penalty_of(const Pen<double>& pn, double den) {
-  const double t = tanh(pn.beta * (den - pn.den_m));
+  const double x = pn.beta * (den - pn.den_m);
+  const float y = (float)(x + x);
+  if (y < -26.0f) return (double)((float)pn.C * expf(y) * (2.0f + 4.0f * (float)pn.beta * (float)den));
+  const double t = tanh(x);
   return pn.C * (1.0 + t + pn.beta * den * (1.0 - t * t));
 }
 EP_DEV float penalty_of(const Pen<float>& pn, float den) {
@@ -199,103 +206,13 @@ EP_DEV T hexp_t(const Phys& ph, C2<T> psi, C2<T> H) {
 // ---------------------------------------------------------------------------
 // X pass helpers (lines along x are contiguous; nl lines per CTA).
 //
-// Half-line transforms of N2 = nx/2 points.  N2 in {16, 32, 64, 128} (and
-// in FP32 also 48, 80, 96) use
-// xlines: P threads of one warp per line, E = N2/P points per thread, the
-// two-factor decomposition of ep_yz.cuh with the exchange done in place in
-// the line's own shared-memory row (stride P+1 for the exchange), fenced by
-// __syncwarp only.  The row stride x_row() makes the step-1 reads, the
-// exchange and the step-2 reads conflict-free for 8- and 16-byte elements.
-// N2 = 0 selects the general shared-memory Stockham engine.
-template <int N2> struct XShape;
-template <> struct XShape<16> { static constexpr int P = 4, E = 4; };
-template <> struct XShape<32> { static constexpr int P = 4, E = 8; };
-template <> struct XShape<64> { static constexpr int P = 8, E = 8; };
-template <> struct XShape<128> { static constexpr int P = 8, E = 16; };
-template <> struct XShape<48> { static constexpr int P = 4, E = 12; };
-template <> struct XShape<80> { static constexpr int P = 4, E = 20; };
-template <> struct XShape<96> { static constexpr int P = 4, E = 24; };
-
-// the register transform length of half-lines of n2 points (0: the general
-// engine); the mixed-radix lengths only in FP32, where the FP64 engine is
-// bound by its arithmetic pipe either way
-template <class T>
-__host__ __device__ constexpr int x_reg_n2(int n2) {
-  // double-float X passes run faster on the general engine (823 against 761
-  // steps/s at 128^3): the register transforms' 4 lines per warp leave half of
-  // a 16-line CTA waiting at its barriers
-  return (!std::is_same<T, dfloat>::value && (n2 == 16 || n2 == 32 || n2 == 64 || n2 == 128)) ? n2
-         : (sizeof(T) == 4 && (n2 == 48 || n2 == 80 || n2 == 96)) ? n2
-                                                                    : 0;
-}
-// row stride (complex elements): >= n2 + 1 and >= E (P + 1), and congruent
-// to P modulo 16 so that the lines sharing a half-warp fall on distinct banks
-__host__ __device__ constexpr int x_row(int n2, int reg) {
-  return !reg ? n2 + 1
-              : (n2 == 16 ? 20 : n2 == 32 ? 52 : n2 == 48 ? 68 : n2 == 64 ? 72 : n2 == 80 ? 100 : n2 == 96 ? 132 : 152);
-}
+// The general engine of the half-line lengths ep_xw.cuh has no kernels for:
+// shared-memory Stockham stages over the CTA's lines.
 // shared memory of an X kernel: two line buffers, the twiddles exp(-2 pi i
-// k/nx), the [ka][t] twiddle table of xlines, nreal real arrays
+// k/nx), nreal real arrays
 template <class T>
 __host__ __device__ constexpr size_t x_smem_bytes(int nl, int nx, int nreal) {
-  return 2 * (size_t)nl * x_row(nx / 2, x_reg_n2<T>(nx / 2)) * sizeof(C2<T>) + (size_t)nx * sizeof(C2<T>) +
-         (size_t)(x_reg_n2<T>(nx / 2) ? nx / 2 : 0) * sizeof(C2<T>) + (size_t)nreal * nl * nx * sizeof(T);
-}
-
-template <class T, int N2, int DIR>
-EP_DEV void xlines(C2<T>* A, int nl, int ld, const C2<T>* __restrict__ twt) {
-  constexpr int P = XShape<N2>::P, E = XShape<N2>::E, LPW = 32 / P, Q = P + 1;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int t = lane % P, lsub = lane / P;
-  for (int base = warp * LPW; base < nl; base += nw * LPW) {
-    const int l = base + lsub;
-    const bool act = l < nl;
-    C2<T>* row = A + (act ? l : 0) * ld;
-    C2<T> v[E];
-#pragma unroll
-    for (int a = 0; a < E; ++a) v[a] = act ? row[t + P * a] : cmk<T>(T(0), T(0));
-    epfft::dft<T, E, DIR>(v);
-    if (t != 0) {
-#pragma unroll
-      for (int ka = 1; ka < E; ++ka) {
-        const C2<T> w = twt[ka * P + t];
-        v[ka] = DIR < 0 ? cmul(v[ka], w) : cmulc(v[ka], w);
-      }
-    }
-    __syncwarp();
-    if (act) {
-#pragma unroll
-      for (int ka = 0; ka < E; ++ka) row[ka * Q + t] = v[ka];
-    }
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < E / P; ++j) {
-      C2<T> u[P];
-#pragma unroll
-      for (int tt = 0; tt < P; ++tt) u[tt] = row[(t + P * j) * Q + tt];
-      epfft::dft<T, P, DIR>(u);
-#pragma unroll
-      for (int kt = 0; kt < P; ++kt) v[j + (E / P) * kt] = u[kt];
-    }
-    __syncwarp();
-    if (act) {
-#pragma unroll
-      for (int m = 0; m < E; ++m) row[t + P * m] = v[m];
-    }
-  }
-  __syncthreads();
-}
-
-// Transform nl lines held in A (B: scratch); returns the buffer with the result.
-template <class T, int N2, int DIR>
-EP_DEV const C2<T>* x_lines(C2<T>* A, C2<T>* B, int nl, int ld, const FftPlan& p2, const C2<T>* tw,
-                            const C2<T>* twt) {
-  if constexpr (N2 != 0) {
-    xlines<T, N2, DIR>(A, nl, ld, twt);
-    return A;
-  } else {
-    return epfft::lines<T, DIR>(A, B, nl, ld, p2, tw, 2);
-  }
+  return 2 * (size_t)nl * (nx / 2 + 1) * sizeof(C2<T>) + (size_t)nx * sizeof(C2<T>) + (size_t)nreal * nl * nx * sizeof(T);
 }
 
 // Shared-memory carve-up of the X kernels.
@@ -304,96 +221,24 @@ struct XSmem {
   C2<T>* P;
   C2<T>* Q;
   C2<T>* tw;
-  C2<T>* twt;  // [ka][t] twiddles of xlines
-  T* R;        // nreal arrays of nl*nx
+  T* R;  // nreal arrays of nl*nx
   int ld;
-  EP_DEV XSmem(unsigned char* raw, int nl, int nx, int n2reg) {
-    ld = x_row(nx / 2, n2reg);
+  EP_DEV XSmem(unsigned char* raw, int nl, int nx) {
+    ld = nx / 2 + 1;
     P = reinterpret_cast<C2<T>*>(raw);
     Q = P + nl * ld;
     tw = Q + nl * ld;
-    twt = tw + nx;
-    R = reinterpret_cast<T*>(twt + (n2reg ? nx / 2 : 0));
+    R = reinterpret_cast<T*>(tw + nx);
   }
-  // tw and (for the register transforms) twt from the global table twx;
-  // the caller synchronises before use
-  template <int N2> EP_DEV void load_twiddles(const C2<T>* __restrict__ twx, int nx) {
+  // tw from the global table twx; the caller synchronises before use
+  EP_DEV void load_twiddles(const C2<T>* __restrict__ twx, int nx) {
     for (int i = threadIdx.x; i < nx; i += blockDim.x) tw[i] = twx[i];
-    if constexpr (N2 != 0) {
-      constexpr int P = XShape<N2>::P;
-      for (int i = threadIdx.x; i < N2; i += blockDim.x) {
-        const int ka = i / P, t = i - ka * P;
-        twt[i] = twx[2 * t * ka];
-      }
-    }
   }
 };
 
-// Register-resident c2r of half-lines (N2 > 0): thread t of a line packs
-// Z[k] = A + iB (c2r_pack's algebra) for its own k = t + P a straight from
-// the spectrum in global memory, runs xlines' two steps and writes the real
-// line (x = 2m, 2m+1) to Rout.
-template <class T, int N2>
-EP_DEV void x_inverse_reg(const C2<T>* __restrict__ spec, long long line0, int nlv, int nl, int nx, int nxh,
-                          const XSmem<T>& S, T scale, T* Rout) {
-  constexpr int P = XShape<N2>::P, E = XShape<N2>::E, LPW = 32 / P, Q = P + 1;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int t = lane % P, lsub = lane / P;
-  const C2<T>* tw = S.tw;
-  for (int base = warp * LPW; base < nl; base += nw * LPW) {
-    const int l = base + lsub;
-    const bool act = l < nlv;
-    const C2<T>* X = spec + (line0 + (act ? l : 0)) * nxh;
-    C2<T> v[E];
-#pragma unroll
-    for (int a = 0; a < E; ++a) {
-      const int k = t + P * a;
-      const C2<T> xk = act ? X[k] : cmk<T>(T(0), T(0));
-      const C2<T> xc = act ? conjg(X[N2 - k]) : cmk<T>(T(0), T(0));
-      const C2<T> A = xk + xc;
-      const C2<T> B = cmulc(xk - xc, tw[k]);
-      v[a] = A + mul_i(B);
-    }
-    epfft::dft<T, E, +1>(v);
-    if (t != 0) {
-#pragma unroll
-      for (int ka = 1; ka < E; ++ka) v[ka] = cmulc(v[ka], S.twt[ka * P + t]);
-    }
-    C2<T>* row = S.P + (l < nl ? l : 0) * S.ld;
-    __syncwarp();
-    if (l < nl) {
-#pragma unroll
-      for (int ka = 0; ka < E; ++ka) row[ka * Q + t] = v[ka];
-    }
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < E / P; ++j) {
-      C2<T> u[P];
-#pragma unroll
-      for (int tt = 0; tt < P; ++tt) u[tt] = row[(t + P * j) * Q + tt];
-      epfft::dft<T, P, +1>(u);
-#pragma unroll
-      for (int kt = 0; kt < P; ++kt) v[j + (E / P) * kt] = u[kt];
-    }
-    __syncwarp();
-    if (l < nl) {
-#pragma unroll
-      for (int m = 0; m < E; ++m) {
-        const int i = t + P * m;
-        *reinterpret_cast<C2<T>*>(Rout + l * nx + 2 * i) = cmk<T>(v[m].x * scale, v[m].y * scale);
-      }
-    }
-  }
-  __syncthreads();
-}
-
-template <class T, int N2>
+template <class T>
 EP_DEV void x_inverse(const C2<T>* __restrict__ spec, long long line0, int nlv, int nl, int nx, int nxh,
                       const XSmem<T>& S, const FftPlan& p2, T scale, T* Rout) {
-  if constexpr (N2 != 0) {
-    x_inverse_reg<T, N2>(spec, line0, nlv, nl, nx, nxh, S, scale, Rout);
-    return;
-  }
   const int n2 = nx / 2, ld = S.ld;
   C2<T>* P = S.P;
   C2<T>* Q = S.Q;
@@ -406,7 +251,7 @@ EP_DEV void x_inverse(const C2<T>* __restrict__ spec, long long line0, int nlv, 
   __syncthreads();
   epfft::c2r_pack<T>(P, ld, Q, ld, nl, n2, S.tw);
   __syncthreads();
-  const C2<T>* z = x_lines<T, N2, +1>(Q, P, nl, ld, p2, S.tw, S.twt);
+  const C2<T>* z = epfft::lines<T, +1>(Q, P, nl, ld, p2, S.tw, 2);
   for (int e = threadIdx.x; e < nl * n2; e += blockDim.x) {
     int m;
     const int l = epfft::fdivmod(e, n2, inv2, m);
@@ -473,95 +318,11 @@ EP_DEV C2<T> ld2(const T* p) {
   return *reinterpret_cast<const C2<T>*>(p);
 }
 
-// Register-resident r2c of half-lines (N2 > 0): thread t packs its own
-// z[m] = val(2m) + i val(2m+1) = pair(l, m), m = t + P a (one vector load
-// per element from the caller's arrays, all issued before the transform),
-// runs xlines' two steps, fetches
-// the partner Z[N2 - k] of each of its outputs with a warp shuffle (lane
-// P - t, register E - 1 - m; thread 0 holds its own partners) and writes
-// r2c_unpack's X[k] straight to global memory (thread 0 also X[N2]).
-template <class T, int N2, class F>
-EP_DEV void x_forward_reg(F pair, C2<T>* __restrict__ out, long long line0, int nlv, int nl, int nxh,
-                          const XSmem<T>& S) {
-  constexpr int P = XShape<N2>::P, E = XShape<N2>::E, LPW = 32 / P, Q = P + 1;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int t = lane % P, lsub = lane / P;
-  const int plane = lane - t + (P - t) % P;
-  const C2<T>* tw = S.tw;
-  for (int base = warp * LPW; base < nl; base += nw * LPW) {
-    const int l = base + lsub;
-    const bool act = l < nlv;
-    C2<T> v[E];
-#pragma unroll
-    for (int a = 0; a < E; ++a) {
-      const int m = t + P * a;
-      v[a] = act ? pair(l, m) : cmk<T>(T(0), T(0));
-    }
-    epfft::dft<T, E, -1>(v);
-    if (t != 0) {
-#pragma unroll
-      for (int ka = 1; ka < E; ++ka) v[ka] = cmul(v[ka], S.twt[ka * P + t]);
-    }
-    C2<T>* row = S.P + (l < nl ? l : 0) * S.ld;
-    __syncwarp();
-    if (l < nl) {
-#pragma unroll
-      for (int ka = 0; ka < E; ++ka) row[ka * Q + t] = v[ka];
-    }
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < E / P; ++j) {
-      C2<T> u[P];
-#pragma unroll
-      for (int tt = 0; tt < P; ++tt) u[tt] = row[(t + P * j) * Q + tt];
-      epfft::dft<T, P, -1>(u);
-#pragma unroll
-      for (int kt = 0; kt < P; ++kt) v[j + (E / P) * kt] = u[kt];
-    }
-    __syncwarp();
-    // v[m] = Z[t + P m]; w[m] = Z[(N2 - t - P m) mod N2]
-    C2<T> w[E];
-#pragma unroll
-    for (int j = 0; j < E; ++j) {
-      C2<T> u;
-      u.x = __shfl_sync(0xffffffffu, v[j].x, plane);
-      u.y = __shfl_sync(0xffffffffu, v[j].y, plane);
-      w[E - 1 - j] = u;
-    }
-    if (t == 0) {
-#pragma unroll
-      for (int m = 0; m < E; ++m) w[m] = v[(E - m) % E];
-    }
-    if (act) {
-      C2<T>* o = out + (line0 + l) * nxh;
-#pragma unroll
-      for (int m = 0; m < E; ++m) {
-        const int k = t + P * m;
-        const C2<T> zk = v[m], zc = conjg(w[m]);
-        const C2<T> e = epfft::K<T>::half * (zk + zc);
-        const C2<T> od = epfft::K<T>::half * mul_mi(zk - zc);
-        o[k] = e + cmul(tw[k], od);
-      }
-      if (t == 0) {
-        const C2<T> zk = v[0], zc = conjg(v[0]);
-        const C2<T> e = epfft::K<T>::half * (zk + zc);
-        const C2<T> od = epfft::K<T>::half * mul_mi(zk - zc);
-        o[N2] = e + cmul(tw[N2], od);
-      }
-    }
-  }
-  __syncthreads();
-}
-
 // Forward r2c of nl x-lines whose values are pair(l, m) = (val(l, 2m),
 // val(l, 2m+1)).
-template <class T, int N2, class F>
+template <class T, class F>
 EP_DEV void x_forward(F pair, C2<T>* __restrict__ out, long long line0, int nlv, int nl, int nx, int nxh,
                       const XSmem<T>& S, const FftPlan& p2) {
-  if constexpr (N2 != 0) {
-    x_forward_reg<T, N2>(pair, out, line0, nlv, nl, nxh, S);
-    return;
-  }
   const int n2 = nx / 2, ld = S.ld;
   C2<T>* P = S.P;
   const float inv2 = 1.0f / (float)n2;
@@ -571,7 +332,7 @@ EP_DEV void x_forward(F pair, C2<T>* __restrict__ out, long long line0, int nlv,
     P[l * ld + m] = l < nlv ? pair(l, m) : cmk<T>(T(0), T(0));
   }
   __syncthreads();
-  const C2<T>* Z = x_lines<T, N2, -1>(P, S.Q, nl, ld, p2, S.tw, S.twt);
+  const C2<T>* Z = epfft::lines<T, -1>(P, S.Q, nl, ld, p2, S.tw, 2);
   epfft::r2c_unpack<T>(Z, nl, ld, n2, S.tw, [&](int l, int k, C2<T> v) {
     if (l < nlv) out[(line0 + l) * nxh + k] = v;
   });
@@ -579,18 +340,18 @@ EP_DEV void x_forward(F pair, C2<T>* __restrict__ out, long long line0, int nlv,
 }
 
 // X1: den -> r2c along x (-> out).  grad den is k_d1march<MODE 0>.
-template <class T, int N2>
+template <class T>
 __global__ void k_x1(Geo g, const T* __restrict__ den, C2<T>* __restrict__ out, const __grid_constant__ FftPlan p2,
                      const C2<T>* __restrict__ twx, int nl) {
   extern __shared__ __align__(16) unsigned char smraw[];
   const int nx = g.nx;
-  XSmem<T> S(smraw, nl, nx, N2);
+  XSmem<T> S(smraw, nl, nx);
   const long long nlines = (long long)g.ny * g.nz;
   const long long line0 = (long long)blockIdx.x * nl;
   const int nlv = (int)min((long long)nl, nlines - line0);
-  S.template load_twiddles<N2>(twx, nx);
+  S.load_twiddles(twx, nx);
   __syncthreads();
-  x_forward<T, N2>([&](int l, int m) { return ld2(den + (line0 + l) * nx + 2 * m); }, out, line0, nlv, nl, nx,
+  x_forward<T>([&](int l, int m) { return ld2(den + (line0 + l) * nx + 2 * m); }, out, line0, nlv, nl, nx,
                    g.nxh, S, p2);
 }
 
@@ -598,7 +359,7 @@ __global__ void k_x1(Geo g, const T* __restrict__ den, C2<T>* __restrict__ out, 
 // OTC); pot4 partial = delj4 + dencg^2 (a0 + a1 dencg) (poten.f90:34-92);
 // forward r2c of den*dencg*(cp4 + cpp4*dencg) (poten.f90:62-67) and, for
 // OTC, of f*grad(den), f = 1 - denalf/den0s (term_alfa.f90:157-170).
-template <class T, int N2>
+template <class T>
 __global__ void k_x2(Geo g, Phys ph, const C2<T>* __restrict__ B0, const C2<T>* __restrict__ B1,
                      const C2<T>* __restrict__ B2, const T* __restrict__ den, const T* __restrict__ dxd,
                      const T* __restrict__ dyd, const T* __restrict__ dzd, T* __restrict__ dencg,
@@ -606,21 +367,21 @@ __global__ void k_x2(Geo g, Phys ph, const C2<T>* __restrict__ B0, const C2<T>* 
                      C2<T>* C2o, C2<T>* C3, const __grid_constant__ FftPlan p2, const C2<T>* __restrict__ twx, int nl) {
   extern __shared__ __align__(16) unsigned char smraw[];
   const int nx = g.nx, nxh = g.nxh;
-  XSmem<T> S(smraw, nl, nx, N2);
+  XSmem<T> S(smraw, nl, nx);
   const bool otc = (ph.core == 1);
   const long long nlines = (long long)g.ny * g.nz;
   const long long line0 = (long long)blockIdx.x * nl;
   const int nlv = (int)min((long long)nl, nlines - line0);
-  S.template load_twiddles<N2>(twx, nx);
+  S.load_twiddles(twx, nx);
   __syncthreads();
   T* Rcg = S.R;
   T* Rlj = S.R + nl * nx;
   T* Ral = S.R + 2 * nl * nx;
   const PConst<T> kc(ph);
   const T rn = kc.renor;
-  x_inverse<T, N2>(B0, line0, nlv, nl, nx, nxh, S, p2, rn, Rcg);
-  x_inverse<T, N2>(B1, line0, nlv, nl, nx, nxh, S, p2, rn, Rlj);
-  if (otc) x_inverse<T, N2>(B2, line0, nlv, nl, nx, nxh, S, p2, rn, Ral);
+  x_inverse<T>(B0, line0, nlv, nl, nx, nxh, S, p2, rn, Rcg);
+  x_inverse<T>(B1, line0, nlv, nl, nx, nxh, S, p2, rn, Rlj);
+  if (otc) x_inverse<T>(B2, line0, nlv, nl, nx, nxh, S, p2, rn, Ral);
   const T a0 = kc.a0, a1 = kc.a1, rden0s = kc.rden0s, cp4 = kc.cp4, cpp4 = kc.cpp4;
   const bool vec = nx % (16 / (int)sizeof(T)) == 0;
   pointwise<T>(nlv * nx, vec, [&](int e, auto kc) {
@@ -642,7 +403,7 @@ __global__ void k_x2(Geo g, Phys ph, const C2<T>* __restrict__ B0, const C2<T>* 
     }
   });
   __syncthreads();
-  x_forward<T, N2>(
+  x_forward<T>(
       [&](int l, int m) {
         const C2<T> cg = ld2(Rcg + l * nx + 2 * m), d = ld2(den + (line0 + l) * nx + 2 * m);
         return cmk<T>(d.x * cg.x * (cp4 + cpp4 * cg.x), d.y * cg.y * (cp4 + cpp4 * cg.y));
@@ -655,7 +416,7 @@ __global__ void k_x2(Geo g, Phys ph, const C2<T>* __restrict__ B0, const C2<T>* 
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const T* gc = grad[c];
-      x_forward<T, N2>(
+      x_forward<T>(
           [&](int l, int m) {
             const C2<T> f = ld2(Ral + l * nx + 2 * m), d = ld2(gc + (line0 + l) * nx + 2 * m);
             return cmk<T>(f.x * d.x, f.y * d.y);
@@ -669,7 +430,7 @@ __global__ void k_x2(Geo g, Phys ph, const C2<T>* __restrict__ B0, const C2<T>* 
 // poten.f90:74,88-92,122-126).  OTC: c2r of the three alpha_s integrals
 // (term_alfa.f90:172-181), the x-derivative of f*I_x, f*I_y and f*I_z for
 // the divergence (:216-225), and forward r2c of grad(den).I (:194-201).
-template <class T, int N2>
+template <class T>
 __global__ void k_x3(Geo g, Phys ph, const __grid_constant__ FdW<T> fd, const C2<T>* __restrict__ D0, const C2<T>* __restrict__ D1,
                      const C2<T>* __restrict__ D2, const C2<T>* __restrict__ D3, const T* __restrict__ den,
                      const T* __restrict__ dxd, const T* __restrict__ dyd, const T* __restrict__ dzd,
@@ -678,16 +439,16 @@ __global__ void k_x3(Geo g, Phys ph, const __grid_constant__ FdW<T> fd, const C2
                      C2<T>* E0, const __grid_constant__ FftPlan p2, const C2<T>* __restrict__ twx, int nl) {
   extern __shared__ __align__(16) unsigned char smraw[];
   const int nx = g.nx, nxh = g.nxh;
-  XSmem<T> S(smraw, nl, nx, N2);
+  XSmem<T> S(smraw, nl, nx);
   const bool otc = (ph.core == 1);
   const long long nlines = (long long)g.ny * g.nz;
   const long long line0 = (long long)blockIdx.x * nl;
   const int nlv = (int)min((long long)nl, nlines - line0);
-  S.template load_twiddles<N2>(twx, nx);
+  S.load_twiddles(twx, nx);
   __syncthreads();
   const T rn = PConst<T>(ph).renor;
   T* Rc = S.R;
-  x_inverse<T, N2>(D0, line0, nlv, nl, nx, nxh, S, p2, rn, Rc);
+  x_inverse<T>(D0, line0, nlv, nl, nx, nxh, S, p2, rn, Rc);
   if (!otc) {
     const Pen<T> pn(ph);
     pointwise<T>(nlv * nx, nx % (16 / (int)sizeof(T)) == 0, [&](int e, auto kc) {
@@ -704,9 +465,9 @@ __global__ void k_x3(Geo g, Phys ph, const __grid_constant__ FdW<T> fd, const C2
   T* Rx = S.R + nl * nx;
   T* Ry = S.R + 2 * nl * nx;
   T* Rz = S.R + 3 * nl * nx;
-  x_inverse<T, N2>(D1, line0, nlv, nl, nx, nxh, S, p2, rn, Rx);
-  x_inverse<T, N2>(D2, line0, nlv, nl, nx, nxh, S, p2, rn, Ry);
-  x_inverse<T, N2>(D3, line0, nlv, nl, nx, nxh, S, p2, rn, Rz);
+  x_inverse<T>(D1, line0, nlv, nl, nx, nxh, S, p2, rn, Rx);
+  x_inverse<T>(D2, line0, nlv, nl, nx, nxh, S, p2, rn, Ry);
+  x_inverse<T>(D3, line0, nlv, nl, nx, nxh, S, p2, rn, Rz);
   pointwise<T>(nlv * nx, nx % (16 / (int)sizeof(T)) == 0, [&](int e, auto kc) {
     constexpr int K = decltype(kc)::value;
     const long long p = line0 * nx + e;
@@ -735,7 +496,7 @@ __global__ void k_x3(Geo g, Phys ph, const __grid_constant__ FdW<T> fd, const C2
       const int l = epfft::fdivmod(e, nx, 1.0f / (float)nx, i);
     dgx[line0 * nx + e] = d1_line(Rc + l * nx, i, nx, fd.w1[0], fd.R, fd.periodic);
   }
-  x_forward<T, N2>(
+  x_forward<T>(
       [&](int l, int m) {
         const int e = l * nx + 2 * m;
         const long long p = line0 * nx + e;
@@ -748,21 +509,21 @@ __global__ void k_x3(Geo g, Phys ph, const __grid_constant__ FdW<T> fd, const C2
 
 // X4 (OTC): c2r of kalfs*FFT(grad(den).I) -> U_alpha = (u/den0s + div(f I))
 // * h2o2m4 * alphas (term_alfa.f90:203-236); pot4 += U_alpha + penalty.
-template <class T, int N2>
+template <class T>
 __global__ void k_x4(Geo g, Phys ph, const C2<T>* __restrict__ F0, const T* __restrict__ den,
                      const T* __restrict__ dgx, const T* __restrict__ dyz, T* __restrict__ pot4,
                      T* __restrict__ ualphas, const __grid_constant__ FftPlan p2, const C2<T>* __restrict__ twx, int nl) {
   extern __shared__ __align__(16) unsigned char smraw[];
   const int nx = g.nx, nxh = g.nxh;
-  XSmem<T> S(smraw, nl, nx, N2);
+  XSmem<T> S(smraw, nl, nx);
   const long long nlines = (long long)g.ny * g.nz;
   const long long line0 = (long long)blockIdx.x * nl;
   const int nlv = (int)min((long long)nl, nlines - line0);
-  S.template load_twiddles<N2>(twx, nx);
+  S.load_twiddles(twx, nx);
   __syncthreads();
   T* Ru = S.R;
   const PConst<T> kc(ph);
-  x_inverse<T, N2>(F0, line0, nlv, nl, nx, nxh, S, p2, kc.renor, Ru);
+  x_inverse<T>(F0, line0, nlv, nl, nx, nxh, S, p2, kc.renor, Ru);
   const T rden0s = kc.rden0s, h2 = kc.h2o2m4, al = kc.alphas;
   const Pen<T> pn(ph);
   pointwise<T>(nlv * nx, nx % (16 / (int)sizeof(T)) == 0, [&](int e, auto kc) {

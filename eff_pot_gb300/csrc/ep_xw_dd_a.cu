@@ -1,0 +1,4 @@
+// ep_xw_dd_a.cu - X pass kernels, part a of the half-line lengths, for dfloat fields.
+#include "ep_xw.cuh"
+EP_XW_PART(xw_part_a, EP_XW_LENGTHS_A)
+template const XWKernels* xw_part_a<dfloat>(int);

@@ -1,0 +1,4 @@
+// ep_xw_fp64_d.cu - X pass kernels, part d of the half-line lengths, for double fields.
+#include "ep_xw.cuh"
+EP_XW_PART(xw_part_d, EP_XW_LENGTHS_D)
+template const XWKernels* xw_part_d<double>(int);

@@ -77,8 +77,9 @@ template <class T, int A, int B> struct YZ {
   // Lines per CTA: 32 in FP32 (256-byte runs) while their buffer stays within
   // 42 KB, else 16 (the two measure alike on one 128^3 instance and 32 is 5 %
   // faster in a batch); 16 of the 16-byte values (32 leave a 64 x 64 x 80 grid
-  // on 66 CTAs: Z 58 us against 45), 8 where two buffers of 16 would not fit.
-  static constexpr int LL = sizeof(T) == 4 ? (32 * N * 8 <= 42 * 1024 ? 32 : 16) : (N <= 256 ? 16 : 8);
+  // on 66 CTAs: Z 58 us against 45), 8 up to 72 points, whose grids are small,
+  // and where two buffers of 16 would not fit.
+  static constexpr int LL = sizeof(T) == 4 ? (32 * N * 8 <= 42 * 1024 ? 32 : 16) : (N > 72 && N <= 256 ? 16 : 8);
   // Slots per line: the count with the largest share of busy slots over the
   // column and row rounds, less 5 to 16 % below eight slots (fewer loads in
   // flight) and 4 % where the CTA is no whole number of warps.
