@@ -147,6 +147,16 @@ bool graph_valid(const StepGraph& G, const std::vector<ep_ctx*>& cs) {
   return true;
 }
 
+// Marks the steps of cs as lean (Engine::lean) for the scope's life.
+struct LeanSteps {
+  const std::vector<ep_ctx*>& cs;
+  explicit LeanSteps(const std::vector<ep_ctx*>& c) : cs(c) { set(true); }
+  ~LeanSteps() { set(false); }
+  void set(bool on) const {
+    for (ep_ctx* c : cs) dispatch(c, [&](auto& e) -> int { e.lean = on; return EP_OK; });
+  }
+};
+
 // Every instance stream waits for the batch stream, then the batch stream
 // waits for every instance: batch events bracket all instances' work.
 void batch_fork(ep_batch* b) {
@@ -303,7 +313,7 @@ int replay_steps(StepGraph& G, const std::vector<ep_ctx*>& cs, cudaStream_t st) 
   return EP_OK;
 }
 
-// ng graph-eligible steps of every context of cs: whole rotation periods
+// ng graph-eligible (and lean) steps of every context of cs: whole rotation periods
 // from the multi-step graph Gk (captured at the first phase that needs it),
 // the rest -- realignment and remainder -- as single replayed steps of G1.
 int graph_steps(StepGraph& G1, StepGraph& Gk, const std::vector<ep_ctx*>& cs, cudaStream_t st, ep_batch* b,
@@ -777,23 +787,30 @@ int ep_steppc(ep_ctx* c, double dt, ep_step_errors* err) {
 
 int ep_run(ep_ctx* c, int nsteps, double dt, ep_run_stats* stats) {
   if (!c || nsteps < 0) return EP_ERR_INVALID_ARG;
-  const bool renorm = c->cfg.time_mode == EP_IMAGINARY_TIME && c->cfg.renormalize;
+  const std::vector<ep_ctx*> one{c};
   int s0 = 0;
-  const int ng = nsteps - (stats ? 1 : 0);  // steps that need no host statistics
-  if (ng >= 2 && graph_eligible(c)) {
-    std::vector<ep_ctx*> one{c};
+  // every step but the last: no statistics, and no field of it outlives it
+  const int ng = nsteps - 1;
+  if (ng > 0) {
+    const LeanSteps lean(one);
     int r;
-    if ((r = graph_steps(c->graph, c->graphk, one, c->st, nullptr, dt, ng, c->use_graphs))) return r;
-    s0 = ng;
+    if (ng >= 2 && graph_eligible(c)) {
+      if ((r = graph_steps(c->graph, c->graphk, one, c->st, nullptr, dt, ng, c->use_graphs))) return r;
+      s0 = ng;
+    }
+    r = dispatch(c, [&](auto& e) -> int {
+      for (; s0 < ng; ++s0)
+        if (int q = e.steppc(dt, nullptr)) return q;
+      return EP_OK;
+    });
+    if (r) return r;
   }
   return dispatch(c, [&](auto& e) -> int {
     ep_step_errors se{};
-    for (int s = s0; s < nsteps; ++s) {
-      const bool last = (s == nsteps - 1) && stats;
-      int r = e.steppc(dt, last ? &se : nullptr);
+    if (nsteps > 0) {
+      int r = e.steppc(dt, stats ? &se : nullptr);
       if (r) return r;
     }
-    (void)renorm;
     if (stats) {
       stats->errHe = se.errHe;
       stats->mu = e.last_mu;
@@ -878,10 +895,12 @@ int ep_batch_run(ep_batch* b, int nsteps, double dt, ep_run_stats* stats) {
   cudaSetDevice(b->device);
   batch_join(b);  // work the caller left on the instance streams comes first
   int s0 = 0;
-  const int ng = nsteps - (stats ? 1 : 0);
+  // every step but the last: no statistics, and no field of it outlives it
+  const int ng = nsteps - 1;
   bool eligible = b->use_graphs > 0 && ng >= 2;
   for (ep_ctx* c : b->ctx) eligible = eligible && graph_eligible(c);
   if (eligible) {
+    const LeanSteps lean(b->ctx);
     int r;
     if ((r = graph_steps(b->graph, b->graphk, b->ctx, b->st, b, dt, ng, b->use_graphs))) return r;
     s0 = ng;
@@ -889,15 +908,14 @@ int ep_batch_run(ep_batch* b, int nsteps, double dt, ep_run_stats* stats) {
   batch_fork(b);
   // step-major interleaving so the instances' kernels overlap
   for (int s = s0; s < nsteps; ++s) {
-    const bool last = (s == nsteps - 1) && stats;
+    const bool final = s == nsteps - 1, last = final && stats;
     for (size_t i = 0; i < b->ctx.size(); ++i) {
-      ep_ctx* c = b->ctx[i];
-      const bool renorm = c->cfg.time_mode == EP_IMAGINARY_TIME && c->cfg.renormalize;
       ep_step_errors se{};
-      int r = dispatch(c, [&](auto& e) -> int {
+      int r = dispatch(b->ctx[i], [&](auto& e) -> int {
+        e.lean = !final;
         int q = e.steppc(dt, last ? &se : nullptr);
+        e.lean = false;
         if (q) return q;
-        (void)renorm;
         if (last) {
           stats[i].errHe = se.errHe;
           stats[i].mu = e.last_mu;

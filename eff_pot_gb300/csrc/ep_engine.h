@@ -216,6 +216,12 @@ class Engine {
   // Apply the lazy renormalisation scales before host-visible operations.
   int ensure_materialized();
   bool lazy = false;
+  // A step whose fields the next step of the same call overwrites before the
+  // caller can read them: the fields that only energy() and the downloads read
+  // (dencg, delj4, I_xyz, U_alpha; with frozen internal variables the impurity's
+  // V_Pi, Delta and moments) are not stored.  ep_run and ep_batch_run set it for
+  // all but their last step.
+  bool lean = false;
   CT* slot_base[EP_NSLOTS] = {};
 
   // precision conversion (the other engine's state -> this one)
@@ -230,7 +236,10 @@ class Engine {
   int rk_stage(int jr, double dt);
   int reduce_finalize(int nblocks, int nq, int out0, int mode);
   int read_sums(double* h, int n, int off);
-  dim3 col_grid(ColGrid& cg) const;
+  dim3 col_grid(ColGrid& cg, int sum_rows) const;
+  // a lean step of a P-state impurity with frozen internal variables needs the
+  // force alone
+  bool force_only() const { return lean && cfg.fix_lambda && cfg.state == EP_STATE_P; }
   int fft_y(CT** arrs, int n, int dir);
   int yz_launch(const char* name, const void* fn, const YZKernels& k, size_t smem, const LineSet& ls, int n,
                 void** args);

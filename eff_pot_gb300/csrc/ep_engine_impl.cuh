@@ -476,13 +476,14 @@ int Engine<T>::potenimp() {
       float2 fv[6];
       for (int i = 0; i < 6; ++i) fv[i] = make_float2((float)imp->invar[i].real(), (float)imp->invar[i].imag());
       const double h = rmax / (imp->npot - 1);
+      T *vp = force_only() ? nullptr : vpi, *dl = force_only() ? nullptr : delta;
       ColGrid cg;
-      const dim3 grid = col_grid(cg);
+      const dim3 grid = col_grid(cg, 0);
       auto kf = k_potenimp_f;
       EP_LAUNCH("potenimp", kf, grid, dim3(32, 8), cg.rows * sizeof(float), g, cg, cfg.xmax, cfg.ymax, cfg.zmax, hx,
                 hy, hz, imp->rimp[0], imp->rimp[1], imp->rimp[2], imp->d_potpi_f,
                 imp->d_potdel_f, imp->npot, (float)h, (float)(1.0 / h), (float)imp->umax_sigma, fv[0], fv[1], fv[2],
-                fv[3], fv[4], fv[5], vpi, delta, uimp);
+                fv[3], fv[4], fv[5], vp, dl, uimp);
       return EP_OK;
     }
   }
@@ -491,23 +492,38 @@ int Engine<T>::potenimp() {
     for (int i = 0; i < 6; ++i) iv[i] = make_double2(imp->invar[i].real(), imp->invar[i].imag());
     const double h = rmax / (imp->npot - 1);
     const ImpTable tab{imp->d_coef, imp->npot, h, 1.0 / h, imp->umax_sigma};
+    T *vp = force_only() ? nullptr : vpi, *dl = force_only() ? nullptr : delta;
     ColGrid cg;
-    const dim3 grid = col_grid(cg);
+    const dim3 grid = col_grid(cg, 0);
     auto k = k_potenimp<T>;
     EP_LAUNCH("potenimp", k, grid, dim3(32, 8), cg.rows * sizeof(double2), g, cg, cfg.xmax, cfg.ymax, cfg.zmax, hx, hy, hz, imp->rimp[0],
-              imp->rimp[1], imp->rimp[2], tab, iv[0], iv[1], iv[2], iv[3], iv[4], iv[5], vpi, delta, uimp);
+              imp->rimp[1], imp->rimp[2], tab, iv[0], iv[1], iv[2], iv[3], iv[4], iv[5], vp, dl, uimp);
   }
   return EP_OK;
 }
 
-// Launch grid of the column kernels: groups of 32 columns by chunks of rows,
-// at least three CTAs per SM where the grid allows (an FP64-bound kernel of
-// 160 CTAs would leave 144 SMs idle for half its time), at most EP_RED_BLOCKS
-// in all, the groups spread evenly over the CTAs of a chunk.
+// Launch grid of the column kernels: groups of 32 columns by chunks of rows, at
+// most EP_RED_BLOCKS CTAs in all, the groups spread evenly over a chunk's CTAs.
+// sum_rows: the rows a thread could process in the time of its share of the
+// block reduction (0: a kernel without one).  FP64 sums are bound by each SM's
+// FP64 pipe, so their chunk count minimises CTAs per SM x (rows + sum_rows)
+// (energy, 64 x 64 x 80: 160 CTAs 251 us, 480 191; 64^3: 512 CTAs 151 us, 128
+// 132); the others take about three CTAs per SM where the grid allows.
 template <class T>
-dim3 Engine<T>::col_grid(ColGrid& cg) const {
+dim3 Engine<T>::col_grid(ColGrid& cg, int sum_rows) const {
   cg.groups = (int)(((long long)g.nx * g.nz + 31) / 32);
   int chunks = (3 * dev_sm + cg.groups - 1) / cg.groups;
+  if (sum_rows && std::is_same<T, double>::value) {
+    const int top = std::max(1, std::min(chunks, g.ny / 8));
+    double best = 0.0;
+    for (int c = 1; c <= top; ++c) {
+      const double cost = (double)((cg.groups * c + dev_sm - 1) / dev_sm) * (g.ny / (8.0 * c) + sum_rows);
+      if (c == 1 || cost < best) {
+        best = cost;
+        chunks = c;
+      }
+    }
+  }
   chunks = std::max(1, std::min(chunks, g.ny / 8));
   chunks = std::max(chunks, (g.ny + 2047) / 2048);  // the row tables: 16 bytes a row at most
   cg.rows = (g.ny + chunks - 1) / chunks;
@@ -543,7 +559,7 @@ int Engine<T>::energy(ep_energies* e) {
   for (int i = 0; i < 4; ++i) vp.par[i] = imp->plus.par[i];
   vp.s = imp->plus_series;
   ColGrid cg;
-  const dim3 grid = col_grid(cg);
+  const dim3 grid = col_grid(cg, 2);
   double s[8];
   // W: the arithmetic of the terms (k_energy); mode 3 leaves the flag alone
   auto sums = [&](auto w, int mode) -> int {
@@ -634,14 +650,15 @@ int Engine<T>::forceimp(double* F) {
     return EP_OK;
   }
   ColGrid cg;
-  const dim3 grid = col_grid(cg);
-  auto k = k_impmoments<T>;
+  const dim3 grid = col_grid(cg, 4);
+  const bool force = force_only();
+  auto k = force ? k_impmoments<T, false> : k_impmoments<T, true>;
   EP_LAUNCH("impmoments", k, grid, dim3(32, 8), cg.rows * sizeof(T), g, cg, den, dxd, dyd, dzd, uimp, vpi, delta,
             cfg.xmax, cfg.ymax, cfg.zmax, hx, hy, hz, imp->rimp[0], imp->rimp[1], imp->rimp[2], izlo, izhi, partials);
   int r;
-  if ((r = reduce_finalize((int)(grid.x * grid.y), 9, 16, 0))) return r;
-  double s[9];
-  if ((r = read_sums(s, 9, 16))) return r;
+  if ((r = reduce_finalize((int)(grid.x * grid.y), force ? 3 : 9, 16, 0))) return r;
+  double s[3];
+  if ((r = read_sums(s, 3, 16))) return r;
   for (int i = 0; i < 3; ++i) F[i] = -s[i] * dxyz;
   return EP_OK;
 }
@@ -1393,7 +1410,7 @@ int Engine<T>::x_pass(int which, bool otc) {
   a.intx = intx; a.inty = inty; a.intz = intz; a.gy = gy; a.gz = gz; a.dgx = dgx; a.ualphas = ualphas;
   a.dyz = dyz;
   a.twx = twx;
-  a.keep = 1;
+  a.keep = lean ? 0 : 1;
   void* args[] = {&nlines, &phys, &fd, &a};
   cudaEvent_t ev = nullptr;
   int c = -1;

@@ -88,8 +88,17 @@ struct ImpTable {
   double h, rh;        // spacing and its reciprocal
   double umax_sigma;
 };
+// 1 / sqrt(x) for normal x > 0: the approximate root instruction (about 2^-20)
+// and one third-order correction y += y e (1/2 + 3/8 e), e = 1 - x y^2 (left:
+// 5/16 e^3, below 2^-57), six FP64-pipe operations.
+EP_DEV double fast_rsqrt(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x * y, y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
 EP_DEV void imp_field(const ImpTable& t, double rr2, double& vp, double& dl) {
-  const double rs = rsqrt(rr2);
+  const double rs = fast_rsqrt(rr2);
   double r = rr2 * rs;
   r = fma(fma(-r, r, rr2), 0.5 * rs, r);
   const double q = fma(r, t.rh, 1.5);
@@ -167,9 +176,13 @@ __global__ void __launch_bounds__(256) k_potenimp(Geo g, ColGrid cg, double xmax
         imp_field(t, rr2, vp, dl);
         const double ox = iv2.x * yy + oxc, oy = iv2.y * yy + oyc, ex = iv3.x * yy + exc, ey = iv3.y * yy + eyc;
         const double u = vp + dl * ((ox * ox + oy * oy) + (ex * ex + ey * ey));
-        vpi[p] = to_field<T>(vp);
-        delta[p] = to_field<T>(dl);
-        uimp[p] = to_field<T>(fmin(u, 1000.0));
+        if (vpi) {
+          vpi[p] = to_field<T>(vp);
+          delta[p] = to_field<T>(dl);
+        }
+        // fmin(u, 1000) by the exponent word (0x408f4000: 1000; a NaN gives 1000)
+        const int hu = __double2hiint(u);
+        uimp[p] = to_field<T>(hu < 0x408f4000 && (hu & 0x7ff00000) != 0x7ff00000 ? u : fmin(u, 1000.0));
       },
       [] {});
 }
@@ -319,8 +332,10 @@ static __global__ void __launch_bounds__(256)
         const float ox = iv0.x * xx + iv2.x * yy + iv4.x * zz, oy = iv0.y * xx + iv2.y * yy + iv4.y * zz;
         const float ex = iv1.x * xx + iv3.x * yy + iv5.x * zz, ey = iv1.y * xx + iv3.y * yy + iv5.y * zz;
         const float u = vp + dl * ((ox * ox + oy * oy) + (ex * ex + ey * ey));
-        vpi[p] = vp;
-        delta[p] = dl;
+        if (vpi) {
+          vpi[p] = vp;
+          delta[p] = dl;
+        }
         uimp[p] = fminf(u, 1000.0f);
       },
       [] {});
@@ -355,8 +370,9 @@ EP_DEV float fmul1(float a, float b) { return a * b; }
 // rounding, and the FP64 conversions, products and sums of the one-point form
 // (about 120 operations a point on the FP64 pipe) go: 96 x 160 x 192 896 ->
 // 46 us; FP64 64 x 64 x 80 360 -> 123 us; FP32 256 x 256 x 320
-// 168 -> 120 us (memory: seven fields read).
-template <class T>
+// 168 -> 120 us (memory: seven fields read).  MOM = false: the force alone
+// (three sums, four fields read).
+template <class T, bool MOM>
 __global__ void __launch_bounds__(256) k_impmoments(Geo g, ColGrid cg, const T* __restrict__ den,
                                                     const T* __restrict__ dxd, const T* __restrict__ dyd,
                                                     const T* __restrict__ dzd, const T* __restrict__ uimp,
@@ -375,7 +391,7 @@ __global__ void __launch_bounds__(256) k_impmoments(Geo g, ColGrid cg, const T* 
   for (int i = threadIdx.x + 32 * threadIdx.y; i < cg.rows; i += 32 * blockDim.y)
     ys[i] = T(coord(ymax, hy, y0 + i) - r1);
   __syncthreads();
-  Acc<T> acc[9];
+  Acc<T> acc[MOM ? 9 : 3];
   Acc<T> sv, s0, s1, s2;  // along the column: den V_Pi and den Delta (1, y, y^2)
   T xx = T(0), zz = T(0);
   bool fz = false;
@@ -388,17 +404,20 @@ __global__ void __launch_bounds__(256) k_impmoments(Geo g, ColGrid cg, const T* 
         sv = s0 = s1 = s2 = Acc<T>();
       },
       [&](int iy, long long p) {
-        const T u = uimp[p], a1 = den[p], yy = ys[iy - y0];
+        const T u = uimp[p];
         acc[0].add(mul(dxd[p], u));
         acc[1].add(mul(dyd[p], u));
         if (fz) acc[2].add(mul(dzd[p], u));
-        const T d = mul(a1, delta[p]), dy = mul(d, yy);
-        sv.add(mul(a1, vpi[p]));
-        s0.add(d);
-        s1.add(dy);
-        s2.add(mul(dy, yy));
+        if constexpr (MOM) {
+          const T a1 = den[p], yy = ys[iy - y0], d = mul(a1, delta[p]), dy = mul(d, yy);
+          sv.add(mul(a1, vpi[p]));
+          s0.add(d);
+          s1.add(dy);
+          s2.add(mul(dy, yy));
+        }
       },
       [&] {
+        if constexpr (MOM) {
         const T V = wvalue(sv), D = wvalue(s0), Dx = mul(xx, D), Dz = mul(zz, D), Dy = wvalue(s1);
         acc[3].add(V);
         acc[3].add(mul(xx, Dx));
@@ -409,8 +428,9 @@ __global__ void __launch_bounds__(256) k_impmoments(Geo g, ColGrid cg, const T* 
         acc[7].add(mul(zz, Dy));
         acc[8].add(V);
         acc[8].add(mul(zz, Dz));
+        }
       });
-  block_reduce_store_acc<9>(acc, partials);
+  block_reduce_store_acc<MOM ? 9 : 3>(acc, partials);
 }
 
 // Sum of |psi|^2 (block partials).
