@@ -20,6 +20,8 @@
 
 #include "../../include/eff_pot.h"
 #include "ep_kernels.cuh"
+#include "ep_xw.cuh"
+#include "ep_yz.cuh"
 
 namespace {
 
@@ -27,32 +29,74 @@ namespace {
 // at most 320 points.
 constexpr long long kMaxHalf = 33LL * 64 * 64;
 constexpr int kMaxAxis = 320;
-constexpr long long kScratchElems = 2 * kMaxHalf + 3 * kMaxAxis;
+constexpr long long kScratchElems = 2 * kMaxHalf;
 
 static __device__ __align__(256) double2 g_noalloc_scratch[kScratchElems];
 
 constexpr int kMaxDevices = 64;
 std::mutex g_setup_mutex;
 double2* g_scratch_addr[kMaxDevices] = {};
+const double2* g_roots_addr[kMaxDevices] = {};
 
-// n >= 2 with no prime factor other than 2, 3 and 5 (any length; the
-// scratch limit on the length is checked apart).
-bool axis_ok(int n) {
+// Roots exp(-2 pi i k / n), k < n, of every axis length, as a constant table of
+// the library (89 KB): three kernels a call computed them before, three
+// of eight launches.  With the per-length X, Y and Z kernels a call takes 41 us
+// at 32^3 (57 before) and 51 at 30 x 54 x 64 (78): its five launches.  Each angle is reduced to its octant and the sine or
+// cosine series summed there in long double, then rounded.
+constexpr bool axis_len(int n) {
   if (n < 2) return false;
   while (n % 2 == 0) n /= 2;
   while (n % 3 == 0) n /= 3;
   while (n % 5 == 0) n /= 5;
   return n == 1;
 }
-
-// Roots exp(-2 pi i k / n), k < n.
-__global__ void k_noalloc_twiddles(double2* tw, int n) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    double s, c;
-    sincospi(-2.0 * k / n, &s, &c);
-    tw[k] = make_double2(c, s);
-  }
+constexpr int roots_at(int n) {
+  int at = 0;
+  for (int m = 2; m < n; ++m)
+    if (axis_len(m)) at += m;
+  return at;
 }
+constexpr int kRoots = roots_at(kMaxAxis + 1);
+constexpr long double sin_series(long double x) {
+  long double t = x, s = 0.0L;
+  for (int i = 1; i < 14; ++i) {
+    s += t;
+    t *= -x * x / ((2.0L * i) * (2.0L * i + 1.0L));
+  }
+  return s;
+}
+constexpr long double cos_series(long double x) {
+  long double t = 1.0L, s = 0.0L;
+  for (int i = 1; i < 14; ++i) {
+    s += t;
+    t *= -x * x / ((2.0L * i - 1.0L) * (2.0L * i));
+  }
+  return s;
+}
+struct Roots {
+  double v[2 * kRoots];
+};
+constexpr Roots make_roots() {
+  Roots r{};
+  int at = 0;
+  for (int n = 2; n <= kMaxAxis; ++n) {
+    if (!axis_len(n)) continue;
+    for (int k = 0; k < n; ++k, ++at) {
+      // angle 2 pi k / n = q pi/2 + (pi/2) (f / n), 0 <= f < n
+      const int q = 4 * k / n, f = 4 * k - q * n;
+      const long double half = 1.57079632679489661923132169163975144L;
+      const bool up = 2 * f > n;
+      const long double x = half * (up ? n - f : f) / n;
+      const double a = (double)(up ? sin_series(x) : cos_series(x)), b = (double)(up ? cos_series(x) : sin_series(x));
+      const double co = q == 0 ? a : q == 1 ? -b : q == 2 ? -a : b;
+      const double si = q == 0 ? b : q == 1 ? a : q == 2 ? -b : -a;
+      r.v[2 * at] = co;
+      r.v[2 * at + 1] = -si;
+    }
+  }
+  return r;
+}
+static __device__ const __align__(16) Roots g_noalloc_roots = make_roots();
 
 // Backward c2r along x of every line, scaled by 1/N, into a real array.
 __global__ void k_noalloc_xinv(Geo g, const double2* __restrict__ spec, double* __restrict__ out,
@@ -76,16 +120,19 @@ size_t l_smem_of(int LT, int n, int nbuf) {
   return (size_t)nbuf * LT * (n + 1) * sizeof(double2) + (size_t)n * sizeof(double2) + (size_t)LT * sizeof(long long);
 }
 
-// Once per device, with that device current: the device address of the
-// scratch array and the shared-memory limits of the kernels used here.
-int device_setup(int dev, double2** out) {
+// Once per device, with that device current: the device addresses of the
+// scratch array and the roots and the shared-memory limits of the general
+// kernels.
+int device_setup(int dev, double2** out, const double2** roots) {
   std::lock_guard<std::mutex> lock(g_setup_mutex);
   if (g_scratch_addr[dev]) {
     *out = g_scratch_addr[dev];
+    *roots = g_roots_addr[dev];
     return EP_OK;
   }
-  void* ptr = nullptr;
-  if (cudaGetSymbolAddress(&ptr, g_noalloc_scratch) != cudaSuccess || !ptr) {
+  void *ptr = nullptr, *rp = nullptr;
+  if (cudaGetSymbolAddress(&ptr, g_noalloc_scratch) != cudaSuccess || !ptr ||
+      cudaGetSymbolAddress(&rp, g_noalloc_roots) != cudaSuccess || !rp) {
     cudaGetLastError();
     return EP_ERR_CUDA;
   }
@@ -98,9 +145,21 @@ int device_setup(int dev, double2** out) {
     cudaGetLastError();
     return EP_ERR_CUDA;
   }
+  g_roots_addr[dev] = static_cast<const double2*>(rp);
   g_scratch_addr[dev] = static_cast<double2*>(ptr);
   *out = g_scratch_addr[dev];
+  *roots = g_roots_addr[dev];
   return EP_OK;
+}
+
+// A per-length kernel, whose CTA may want more than the 48 KB default of shared
+// memory.
+cudaError_t launch(const void* fn, dim3 grid, int threads, void** args, size_t smem, cudaStream_t st) {
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaLaunchKernel(fn, grid, dim3((unsigned)threads), args, smem, st);
 }
 
 }  // namespace
@@ -108,7 +167,7 @@ int device_setup(int dev, double2** out) {
 extern "C" int ep_convolve_noalloc(const double* d_in, const double* d_kernel, double* d_out, int nx, int ny,
                                    int nz, void* stream) {
   if (!d_in || !d_kernel || !d_out) return EP_ERR_INVALID_ARG;
-  if (nx % 2 || !axis_ok(nx) || !axis_ok(ny) || !axis_ok(nz)) return EP_ERR_BAD_GRID;
+  if (nx % 2 || !axis_len(nx) || !axis_len(ny) || !axis_len(nz)) return EP_ERR_BAD_GRID;
   const long long half = (long long)(nx / 2 + 1) * ny * nz;
   if (half > kMaxHalf || nx > kMaxAxis || ny > kMaxAxis || nz > kMaxAxis) return EP_ERR_UNSUPPORTED;
   int dev = 0;
@@ -117,45 +176,90 @@ extern "C" int ep_convolve_noalloc(const double* d_in, const double* d_kernel, d
     return EP_ERR_NO_DEVICE;
   }
   double2* scratch = nullptr;
-  int r = device_setup(dev, &scratch);
+  const double2* roots = nullptr;
+  int r = device_setup(dev, &scratch, &roots);
   if (r) return r;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   double2* S = scratch;
   double2* Tsp = scratch + kMaxHalf;
-  double2* twx = scratch + 2 * kMaxHalf;
-  double2* twy = twx + kMaxAxis;
-  double2* twz = twy + kMaxAxis;
-  FftPlan p2{}, pY{}, pZ{};
-  make_plan(nx / 2, p2);
-  make_plan(ny, pY);
-  make_plan(nz, pZ);
+  const double2 *twx = roots + roots_at(nx), *twy = roots + roots_at(ny), *twz = roots + roots_at(nz);
   Geo g{nx, ny, nz, nx / 2 + 1, (long long)nx * ny * nz, half};
-  k_noalloc_twiddles<<<1, 320, 0, st>>>(twx, nx);
-  k_noalloc_twiddles<<<1, 320, 0, st>>>(twy, ny);
-  k_noalloc_twiddles<<<1, 320, 0, st>>>(twz, nz);
-  const long long nlines = (long long)ny * nz;
-  int nl = 16;
-  while (nl > 1 && x_smem_of(nl, nx) > 110 * 1024) nl /= 2;
-  k_x1<double><<<(unsigned)((nlines + nl - 1) / nl), 256, x_smem_of(nl, nx), st>>>(g, d_in, S, p2, twx, nl);
+  long long nlines = (long long)ny * nz;
+  double scale = 1.0 / ((double)nx * ny * nz);
+  cudaError_t e = cudaSuccess;
+  // X forward, Y forward, Z with the product, Y backward, X backward: the
+  // kernels of each axis' length, or the general engine
+  const XWKernels* kx = xw_kernels<double>(nx / 2);
+  const YZKernels *ky = yz_kernels<double>(ny), *kz = yz_kernels<double>(nz);
+  FftPlan p2{}, pY{}, pZ{};
+  int nl = 16, LT = 16, LZ = 16;
+  if (!kx) {
+    make_plan(nx / 2, p2);
+    while (nl > 1 && x_smem_of(nl, nx) > 110 * 1024) nl /= 2;
+  }
+  if (!ky) {
+    make_plan(ny, pY);
+    while (LT > 1 && l_smem_of(LT, ny, 2) > 110 * 1024) LT /= 2;
+  }
+  if (!kz) {
+    make_plan(nz, pZ);
+    while (LZ > 1 && l_smem_of(LZ, nz, 3) > 110 * 1024) LZ /= 2;
+  }
+  const dim3 gx((unsigned)(kx ? (nlines + kx->lines - 1) / kx->lines : (nlines + nl - 1) / nl));
+  if (kx) {
+    Phys ph{};
+    FdW<double> fd{};
+    XWArgs<double> a{};
+    a.den = d_in;
+    a.out[0] = S;
+    a.twx = twx;
+    void* args[] = {&nlines, &ph, &fd, &a};
+    e = launch(kx->x[0], gx, kx->threads, args, kx->smem[0], st);
+  } else {
+    k_x1<double><<<gx, 256, x_smem_of(nl, nx), st>>>(g, d_in, S, p2, twx, nl);
+  }
   Arr8<double> ay{};
-  ay.a[0] = S;
   LineSet ly{(long long)g.nxh, (long long)g.nxh * ny, (long long)g.nxh, (long long)g.nxh * nz};
-  int LT = 16;
-  while (LT > 1 && l_smem_of(LT, ny, 2) > 110 * 1024) LT /= 2;
-  k_c2c<double, -1><<<dim3((unsigned)((ly.nlines + LT - 1) / LT), 1), 256, l_smem_of(LT, ny, 2), st>>>(ay, ly, pY, twy, LT);
+  auto pass_y = [&](double2* a, int dir) {
+    ay.a[0] = a;
+    if (ky) {
+      void* args[] = {&ay, &ly, &twy};
+      if (e == cudaSuccess)
+        e = launch(ky->c2c[dir < 0 ? 0 : 1], dim3((unsigned)((ly.nlines + ky->lines - 1) / ky->lines)), ky->threads,
+                   args, ky->line_bytes + ky->tw_bytes, st);
+      return;
+    }
+    const dim3 grid((unsigned)((ly.nlines + LT - 1) / LT));
+    if (dir < 0) k_c2c<double, -1><<<grid, 256, l_smem_of(LT, ny, 2), st>>>(ay, ly, pY, twy, LT);
+    else k_c2c<double, +1><<<grid, 256, l_smem_of(LT, ny, 2), st>>>(ay, ly, pY, twy, LT);
+  };
+  pass_y(S, -1);
   ConvSpec<double> cs{};
   cs.in[0] = S;
   cs.out[0][0] = Tsp;
   cs.ker[0][0] = d_kernel;
   cs.nout[0] = 1;
   LineSet lz{(long long)g.nxh * ny, 0, (long long)g.nxh * ny, (long long)g.nxh * ny};
-  int LZ = 16;
-  while (LZ > 1 && l_smem_of(LZ, nz, 3) > 110 * 1024) LZ /= 2;
-  k_zconv<double><<<dim3((unsigned)((lz.nlines + LZ - 1) / LZ), 1), 256, l_smem_of(LZ, nz, 3), st>>>(cs, lz, pZ, twz, LZ);
-  ay.a[0] = Tsp;
-  k_c2c<double, +1><<<dim3((unsigned)((ly.nlines + LT - 1) / LT), 1), 256, l_smem_of(LT, ny, 2), st>>>(ay, ly, pY, twy, LT);
-  k_noalloc_xinv<<<(unsigned)((nlines + nl - 1) / nl), 256, x_smem_of(nl, nx), st>>>(
-      g, Tsp, d_out, p2, twx, 1.0 / ((double)nx * ny * nz), nl);
+  if (kz) {
+    void* args[] = {&cs, &lz, &twz};
+    if (e == cudaSuccess)
+      e = launch(kz->conv, dim3((unsigned)((lz.nlines + kz->lines - 1) / kz->lines)), kz->threads, args,
+                 kz->line_bytes + kz->tw_bytes, st);
+  } else {
+    k_zconv<double><<<dim3((unsigned)((lz.nlines + LZ - 1) / LZ)), 256, l_smem_of(LZ, nz, 3), st>>>(cs, lz, pZ, twz, LZ);
+  }
+  pass_y(Tsp, +1);
+  if (kx) {
+    const double2* spec = Tsp;
+    void* args[] = {&nlines, &spec, &d_out, &twx, &scale};
+    if (e == cudaSuccess) e = launch(kx->c2r, gx, kx->threads, args, kx->smem[3], st);
+  } else {
+    k_noalloc_xinv<<<gx, 256, x_smem_of(nl, nx), st>>>(g, Tsp, d_out, p2, twx, scale, nl);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return EP_ERR_CUDA;
+  }
   if (cudaGetLastError() != cudaSuccess) return EP_ERR_CUDA;
   return EP_OK;
 }

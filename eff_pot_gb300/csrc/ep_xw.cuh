@@ -51,6 +51,7 @@ struct XWKernels {
   const void* x[4];
   int lines, threads;  // lines and threads per CTA
   size_t smem[4];
+  const void* c2r;     // FP64 only; shared memory as x[3]
 };
 template <class T> const XWKernels* xw_part_a(int n2);
 template <class T> const XWKernels* xw_part_b(int n2);
@@ -468,13 +469,33 @@ __global__ void __launch_bounds__((XW<T, A, B>::NT), (XW<T, A, B>::MINB))
   });
 }
 
+// c2r alone, scaled, into a real array (ep_convolve_noalloc).
+template <class T, int A, int B>
+__global__ void __launch_bounds__((XW<T, A, B>::NT), (XW<T, A, B>::MINB))
+    k_xw_c2r(long long nlines, const C2<T>* __restrict__ spec, T* __restrict__ out, const C2<T>* __restrict__ twx,
+             T scale) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  XWarp<T, A, B> w(smraw, twx, nlines);
+  w.inverse(spec);
+  w.columns_inverse(scale, [&](int l, int b, C2<T>(&v)[A]) {
+    T* p = out + w.at_field(l, b);
+#pragma unroll
+    for (int i = 0; i < A; ++i) st2(p + 2 * B * i, v[i]);
+  });
+}
+template <class T, int A, int B> const void* xw_c2r() {
+  if constexpr (std::is_same<T, double>::value) return (const void*)k_xw_c2r<T, A, B>;
+  return nullptr;
+}
+
 #define EP_XW_CASE(NN, AA, BB)                                                                                   \
   case NN: {                                                                                                     \
     typedef XW<T, AA, BB> X;                                                                                     \
     static_assert(X::N2 == NN, "factors of the length");                                                         \
     static const XWKernels k{{(const void*)k_xw1<T, AA, BB>, (const void*)k_xw2<T, AA, BB>,                      \
                               (const void*)k_xw3<T, AA, BB>, (const void*)k_xw4<T, AA, BB>},                     \
-                             X::LINES, X::NT, {X::row_bytes(0), X::row_bytes(2), X::row_bytes(3), X::row_bytes(0)}}; \
+                             X::LINES, X::NT, {X::row_bytes(0), X::row_bytes(2), X::row_bytes(3), X::row_bytes(0)}, \
+                             xw_c2r<T, AA, BB>()};                                                               \
     return &k;                                                                                                   \
   }
 #define EP_XW_PART(NAME, LENGTHS)                    \
