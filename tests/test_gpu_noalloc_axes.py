@@ -27,7 +27,7 @@ def test_matches_numpy(dims):
     for p in (0, nx // 2):
         m = ker[:, :, p]
         ker[:, :, p] = 0.5 * (m + np.roll(m[::-1, ::-1], (1, 1), (0, 1)))
-    want = np.fft.irfftn(np.fft.rfftn(a) * ker, s=a.shape)
+    want = np.fft.irfftn(np.fft.rfftn(a) * ker, s=a.shape, axes=(0, 1, 2))
     d_a, d_k = (torch.from_numpy(np.ascontiguousarray(v)).cuda() for v in (a, ker))
     out = torch.empty_like(d_a)
     for _ in range(2):
