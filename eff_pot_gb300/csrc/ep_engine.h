@@ -60,8 +60,9 @@ struct ImpState {
   bool have_tables = false;
 };
 
-// Launch shapes of the FFT passes (lines per CTA and threads per CTA),
-// chosen by Engine::autotune.
+// Launch shapes of the general engine's FFT passes (lines per CTA and threads
+// per CTA), chosen by Engine::autotune; axes with kernels of their own length
+// (ep_xw.cuh, ep_yz.cuh) have theirs fixed.
 struct Shapes {
   int xnl[4] = {16, 16, 16, 16}, xthr[4] = {256, 256, 256, 256};  // X1..X4: x-lines per CTA, threads
   int ylt = 16, ythr = 256;  // Y passes (shared-memory engine)

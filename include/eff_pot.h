@@ -335,7 +335,8 @@ long long ep_batch_kernel_launches(const ep_batch* b);
 
 /* Autotuner: times the poten() pipeline on the current density for
  * candidate launch shapes of the FFT passes (lines and threads per CTA of
- * the X, Y and Z passes) and keeps the fastest.  Needs a density (after
+ * the X, Y and Z passes) and keeps the fastest; axes whose length has kernels of
+ * its own have nothing to tune.  Needs a density (after
  * ep_upload_psi).  report (cap bytes, may be NULL) receives a summary.
  * shapes[6] = {x lines, x threads, y lines, y threads, z lines, z threads}. */
 int ep_autotune(ep_ctx* ctx, char* report, int cap);
