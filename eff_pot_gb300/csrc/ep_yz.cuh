@@ -107,9 +107,8 @@ template <class T, int A, int B> struct YZ {
   static constexpr int REGS = sizeof(T) == 4 ? (A > 16 ? 80 : 64) : (A > 12 ? 168 : 128);
   static constexpr int cap(int m) { return m < 1 ? 1 : (m > 8 ? 8 : m); }
   static constexpr int MINB = cap(65536 / (REGS * NT));
-  // the convolution holds a row's form-factor values too (80 registers: three
-  // CTAs per SM at 128 points, 15.1 us a launch at 128^3 against 15.7 with two)
-  static constexpr int REGS_C = sizeof(T) == 4 ? (A > 16 ? 96 : 80) : REGS;
+  // the convolution holds a row's form-factor values too
+  static constexpr int REGS_C = sizeof(T) == 4 ? (A >= 12 ? 96 : 80) : REGS;
   static constexpr int MINB_C = cap(65536 / (REGS_C * NT));
 };
 
