@@ -124,6 +124,7 @@ _product_only = {
     "select_pot": (_I, [C.c_char_p, C.c_double, C.c_double, C.c_char_p, C.POINTER(EpPotential),
                         C.POINTER(EpSeries), C.c_char_p, _I]),
     "create_error": (C.c_char_p, []),
+    "reset": (_I, [_P]),
     "synchronize": (_I, [_P]),
     "stream": (_P, [_P]),
     "kernel_launches": (C.c_longlong, [_P]),

@@ -674,9 +674,15 @@ int ep_set_impurity_state(ep_ctx* c, const double* rimp, const double* vimp, con
     if (rimp) c->imp.rimp[i] = rimp[i];
     if (vimp) c->imp.vimp[i] = vimp[i];
   }
-  if (invar)
+  if (invar) {
     for (int i = 0; i < 10; ++i) c->imp.invar[i] = std::complex<double>(invar[2 * i], invar[2 * i + 1]);
+    c->imp.new_invar = true;
+  }
   return EP_OK;
+}
+
+int ep_reset(ep_ctx* c) {
+  return dispatch(c, [&](auto& e) -> int { return e.reset_history(); });
 }
 
 int ep_get_impurity_state(ep_ctx* c, double* rimp, double* vimp, double* aimp, double* invar) {

@@ -42,6 +42,26 @@ struct ImpState {
   int ioldr[3] = {0, 1, 2}, ioldv[3] = {0, 1, 2}, iolda[2] = {0, 1}, ioldiv[3] = {0, 1, 2}, ioldhiv[2] = {0, 1};
   double pcr[3] = {0, 0, 0}, pcv[3] = {0, 0, 0};
   std::complex<double> qiv[10], invarold[10][3], hinvarold[10][2], pciv[10];
+  // the internal variables' error estimate of the last steppc, and whether
+  // ep_set_impurity_state has replaced them since (Engine::steprk)
+  double erriv = 0;
+  bool new_invar = false;
+  // Everything a job leaves behind but the state itself (rimp, vimp, invar).
+  void forget() {
+    for (int k = 0; k < 3; ++k) {
+      aimp[k] = qr[k] = qv[k] = pcr[k] = pcv[k] = 0;
+      for (int j = 0; j < 3; ++j) rimpold[k][j] = vimpold[k][j] = 0;
+      for (int j = 0; j < 2; ++j) aimpold[k][j] = 0;
+      ioldr[k] = ioldv[k] = ioldiv[k] = k;
+    }
+    for (int k = 0; k < 10; ++k) {
+      hinvar[k] = qiv[k] = pciv[k] = 0.0;
+      for (int j = 0; j < 3; ++j) invarold[k][j] = 0.0;
+      for (int j = 0; j < 2; ++j) hinvarold[k][j] = 0.0;
+    }
+    for (int k = 0; k < 2; ++k) iolda[k] = ioldhiv[k] = k;
+    erriv = 0;
+  }
   // interpolation tables (module interpol), FP64 on the device
   // P state: d_coef, the parabolas of V_Pi and V_Sigma - V_Pi per interval and
   // side (ImpTable).  D state: d_potdel = V_Delta, d_potpi = V_Pi - V_Delta,
@@ -216,6 +236,7 @@ class Engine {
   int rescale_pending();
   // Apply the lazy renormalisation scales before host-visible operations.
   int ensure_materialized();
+  int reset_history();
   bool lazy = false;
   // A step whose fields the next step of the same call overwrites before the
   // caller can read them: the fields that only energy() and the downloads read

@@ -13,6 +13,7 @@
 
 #define EP_RED_BLOCKS 1216
 #define EP_SMEM_CAP (110 * 1024)
+#define EP_LOST_ERRIV 1e-3
 
 #define EP_LAUNCH(name, kern, grid, block, smem, ...)                 \
   do {                                                                \
@@ -967,9 +968,24 @@ int Engine<T>::rk_stage(int jr, double dt) {
   return EP_OK;
 }
 
-// steprk (steprk.f90:1-191).
 #endif
 #if EP_ENGINE_PARTS & EP_PART_REST
+// The multistep state as ep_create leaves it: psi's history, modifier and
+// Runge-Kutta-Gill carry on the device, the impurity's on the host.  psi, the
+// fields and the impurity's state stay.
+template <class T>
+int Engine<T>::reset_history() {
+  int r;
+  if ((r = ensure_materialized())) return r;
+  for (CT* b : {po[0], po[1], po[2], ph[0], ph[1], pc, q})
+    if ((r = cuda_ok(cudaMemsetAsync(b, 0, g.N * sizeof(CT), st), "reset"))) return r;
+  for (int i = 0; i < 3; ++i) ioldp[i] = i;
+  for (int i = 0; i < 2; ++i) ioldh[i] = i;
+  imp->forget();
+  return EP_OK;
+}
+
+// steprk (steprk.f90:1-191).
 template <class T>
 int Engine<T>::steprk(double dt, bool wait) {
   if (!have_field) { *err = "poten() must run before steprk()"; return EP_ERR_STATE; }
@@ -983,6 +999,16 @@ int Engine<T>::steprk(double dt, bool wait) {
   const double crun[4] = {0.5, 1.0 - 1.0 / s2, 1.0 + 1.0 / s2, 0.5};
   const bool mov = cfg.impurity == EP_IMPURITY_MOVING;
   int r;
+  // New internal variables on a context whose last trajectory of them was
+  // lost.  The method carries its modifiers (p - c) from job to job on a
+  // re-used context, and where dt |H| is large it amplifies them every step
+  // (at 0.1 by 1.17), through all jobs as through one: a 12-step job of an
+  // anisotropic impurity ended in NaN at its 22nd run.  A trajectory whose own
+  // error estimate is beyond EP_LOST_ERRIV a step (of a unit vector; 5e-5 after
+  // such a job's first run) hands nothing on.  Below it the state is carried as
+  // ever; ep_reset starts a job on a re-used context exactly.
+  if (mov && !cfg.fix_lambda && imp->new_invar && !(imp->erriv <= EP_LOST_ERRIV) && (r = reset_history())) return r;
+  imp->new_invar = false;
   for (int jr = 0; jr < 4; ++jr) {
     if ((r = rk_stage(jr, dt))) return r;
     if (mov) {
@@ -1033,6 +1059,7 @@ int Engine<T>::steppc(double dt, ep_step_errors* e) {
   int r;
   if ((r = lap_predict(dt))) return r;
   ImpState& m = *imp;
+  m.new_invar = false;
   if (mov) {
     double auxr[3];
     const int r3 = m.ioldr[2], v1 = m.ioldv[0], v2 = m.ioldv[1], v3 = m.ioldv[2], a1 = m.iolda[0], a2 = m.iolda[1];
@@ -1087,6 +1114,7 @@ int Engine<T>::steppc(double dt, ep_step_errors* e) {
       for (int k = 0; k < nc; ++k) m.invar[k] = auxc[k] + c9 * m.pciv[k];
       for (int k = 0; k < nc; ++k) erriv += std::abs(c9 * m.pciv[k]);
       erriv *= nc == 10 ? 0.1 : 0.1666666666666;
+      m.erriv = erriv;
     }
     { const int t = m.ioldv[2]; m.ioldv[2] = m.ioldv[1]; m.ioldv[1] = m.ioldv[0]; m.ioldv[0] = t; }
     { const int t = m.ioldiv[2]; m.ioldiv[2] = m.ioldiv[1]; m.ioldiv[1] = m.ioldiv[0]; m.ioldiv[0] = t; }

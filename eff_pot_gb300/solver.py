@@ -349,6 +349,11 @@ class Solver:
         parts = names.raw.split(b"\0")
         return {parts[i].decode(): (float(ms[i]), int(cnt[i])) for i in range(min(n.value, maxn))}
 
+    def reset(self):
+        """Clear the multistep state, so that the next job on this context is
+        the one a new context would run (ep_reset)."""
+        self._check(self._f["reset"](self._h), "reset")
+
     # -- convenience: the reference's start-up sequence ---------------------
     def start(self, psi):
         """den=|psi|^2, potenimp, poten (DFT4He3d.f90:436-438)."""

@@ -260,6 +260,16 @@ int ep_set_impurity_state(ep_ctx* ctx, const double* rimp, const double* vimp,
 int ep_get_impurity_state(ep_ctx* ctx, double* rimp, double* vimp,
                           double* aimp, double* invar);
 
+/* Before another job on a context that has run one: clears the multistep state
+ * (psiold, hpsiold, pc, q, the impurity's aimp, histories and modifiers), which
+ * ep_upload_psi and ep_set_impurity_state leave, so that the job is the one a
+ * new context would run, bit for bit.  Without it a job starts from the last
+ * one's modifiers and slopes, as two runs of the reference's subroutines in
+ * one process would -- except that internal variables set anew after their
+ * trajectory was lost (steppc's erriv above 1e-3) start afresh at the next
+ * ep_steprk.  psi, the fields and the impurity's state stay. */
+int ep_reset(ep_ctx* ctx);
+
 /* psi in, den = |psi|^2 (readenc.f90:104-105, DFT4He3d.f90:436). */
 int ep_upload_psi(ep_ctx* ctx, const double* psi);
 int ep_download_psi(ep_ctx* ctx, double* psi);
