@@ -1499,11 +1499,8 @@ int Engine<T>::fft_attrs() {
   cudaFuncSetAttribute(k_c2c<T, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(k_c2c<T, +1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(k_zconv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  if (const YZKernels* k = yz_kernels<T>(g.ny))
-    for (const void* f : k->c2c)
-      cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(k->line_bytes + k->tw_bytes));
-  if (const YZKernels* k = yz_kernels<T>(g.nz))
-    cudaFuncSetAttribute(k->conv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * k->line_bytes + k->tw_bytes));
+  if (const YZKernels* k = yz_kernels<T>(g.ny)) yz_limit_c2c(*k);
+  if (const YZKernels* k = yz_kernels<T>(g.nz)) yz_limit_conv(*k);
   return EP_OK;
 }
 #endif

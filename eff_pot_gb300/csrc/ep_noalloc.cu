@@ -152,15 +152,10 @@ int device_setup(int dev, double2** out, const double2** roots) {
   return EP_OK;
 }
 
-// A per-length kernel, whose CTA may want more than the 48 KB default of shared
-// memory.
 cudaError_t launch(const void* fn, dim3 grid, int threads, void** args, size_t smem, cudaStream_t st) {
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
   return cudaLaunchKernel(fn, grid, dim3((unsigned)threads), args, smem, st);
 }
+constexpr size_t kDefaultSmem = 48 * 1024;  // above it a kernel needs its limit raised
 
 }  // namespace
 
@@ -204,6 +199,13 @@ extern "C" int ep_convolve_noalloc(const double* d_in, const double* d_kernel, d
   if (!kz) {
     make_plan(nz, pZ);
     while (LZ > 1 && l_smem_of(LZ, nz, 3) > 110 * 1024) LZ /= 2;
+  }
+  // (the X kernels' rows stay under the default limit)
+  if (ky && ky->line_bytes + ky->tw_bytes > kDefaultSmem) e = yz_limit_c2c(*ky);
+  if (e == cudaSuccess && kz && kz->line_bytes + kz->tw_bytes > kDefaultSmem) e = yz_limit_conv(*kz);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return EP_ERR_CUDA;
   }
   const dim3 gx((unsigned)(kx ? (nlines + kx->lines - 1) / kx->lines : (nlines + nl - 1) / nl));
   if (kx) {

@@ -484,7 +484,10 @@ __global__ void __launch_bounds__((XW<T, A, B>::NT), (XW<T, A, B>::MINB))
   });
 }
 template <class T, int A, int B> const void* xw_c2r() {
-  if constexpr (std::is_same<T, double>::value) return (const void*)k_xw_c2r<T, A, B>;
+  if constexpr (std::is_same<T, double>::value) {
+    static_assert(XW<T, A, B>::row_bytes(0) <= 48 * 1024, "launched without a raised shared-memory limit");
+    return (const void*)k_xw_c2r<T, A, B>;
+  }
   return nullptr;
 }
 

@@ -72,6 +72,23 @@ template <class T> inline const YZKernels* yz_kernels(int n) {
   return k;
 }
 
+// The limits of dynamic shared memory.  A kernel's limit is its largest use's
+// wherever it is set: contexts and ep_convolve_noalloc launch the same FP64
+// kernels, and a limit lowered to one caller's use (one line buffer of a
+// convolution with one table) refuses the other's launch (two buffers).
+inline cudaError_t yz_limit_c2c(const YZKernels& k) {
+  for (const void* f : k.c2c) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(k.line_bytes + k.tw_bytes));
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+inline cudaError_t yz_limit_conv(const YZKernels& k) {
+  return cudaFuncSetAttribute(k.conv, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)(2 * k.line_bytes + k.tw_bytes));
+}
+
 template <class T, int A, int B> struct YZ {
   static constexpr int N = A * B;
   // Lines per CTA: 32 in FP32 (256-byte runs) while their buffer stays within
