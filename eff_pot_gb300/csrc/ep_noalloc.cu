@@ -16,6 +16,7 @@
 // address is looked up once per device with cudaGetSymbolAddress.
 #include <cuda_runtime.h>
 
+#include <cstdint>
 #include <mutex>
 
 #include "../../include/eff_pot.h"
@@ -162,6 +163,8 @@ constexpr size_t kDefaultSmem = 48 * 1024;  // above it a kernel needs its limit
 extern "C" int ep_convolve_noalloc(const double* d_in, const double* d_kernel, double* d_out, int nx, int ny,
                                    int nz, void* stream) {
   if (!d_in || !d_kernel || !d_out) return EP_ERR_INVALID_ARG;
+  // the X passes read pairs of d_in
+  if ((uintptr_t)d_in % 16 || (uintptr_t)d_kernel % 8 || (uintptr_t)d_out % 8) return EP_ERR_INVALID_ARG;
   if (nx % 2 || !axis_len(nx) || !axis_len(ny) || !axis_len(nz)) return EP_ERR_BAD_GRID;
   const long long half = (long long)(nx / 2 + 1) * ny * nz;
   if (half > kMaxHalf || nx > kMaxAxis || ny > kMaxAxis || nz > kMaxAxis) return EP_ERR_UNSUPPORTED;
@@ -185,10 +188,13 @@ extern "C" int ep_convolve_noalloc(const double* d_in, const double* d_kernel, d
   // X forward, Y forward, Z with the product, Y backward, X backward: the
   // kernels of each axis' length, or the general engine
   const XWKernels* kx = xw_kernels<double>(nx / 2);
+  // k_xw_c2r stores pairs: a d_out that is not 16-byte aligned (a slice of a
+  // host's pool) takes the general engine's last pass, which stores doubles
+  const XWKernels* ko = (uintptr_t)d_out % 16 ? nullptr : kx;
   const YZKernels *ky = yz_kernels<double>(ny), *kz = yz_kernels<double>(nz);
   FftPlan p2{}, pY{}, pZ{};
   int nl = 16, LT = 16, LZ = 16;
-  if (!kx) {
+  if (!kx || !ko) {
     make_plan(nx / 2, p2);
     while (nl > 1 && x_smem_of(nl, nx) > 110 * 1024) nl /= 2;
   }
@@ -207,7 +213,10 @@ extern "C" int ep_convolve_noalloc(const double* d_in, const double* d_kernel, d
     cudaGetLastError();
     return EP_ERR_CUDA;
   }
-  const dim3 gx((unsigned)(kx ? (nlines + kx->lines - 1) / kx->lines : (nlines + nl - 1) / nl));
+  auto grid_x = [&](const XWKernels* k) {
+    const int lines = k ? k->lines : nl;
+    return dim3((unsigned)((nlines + lines - 1) / lines));
+  };
   if (kx) {
     Phys ph{};
     FdW<double> fd{};
@@ -216,9 +225,9 @@ extern "C" int ep_convolve_noalloc(const double* d_in, const double* d_kernel, d
     a.out[0] = S;
     a.twx = twx;
     void* args[] = {&nlines, &ph, &fd, &a};
-    e = launch(kx->x[0], gx, kx->threads, args, kx->smem[0], st);
+    e = launch(kx->x[0], grid_x(kx), kx->threads, args, kx->smem[0], st);
   } else {
-    k_x1<double><<<gx, 256, x_smem_of(nl, nx), st>>>(g, d_in, S, p2, twx, nl);
+    k_x1<double><<<grid_x(nullptr), 256, x_smem_of(nl, nx), st>>>(g, d_in, S, p2, twx, nl);
   }
   Arr8<double> ay{};
   LineSet ly{(long long)g.nxh, (long long)g.nxh * ny, (long long)g.nxh, (long long)g.nxh * nz};
@@ -251,12 +260,12 @@ extern "C" int ep_convolve_noalloc(const double* d_in, const double* d_kernel, d
     k_zconv<double><<<dim3((unsigned)((lz.nlines + LZ - 1) / LZ)), 256, l_smem_of(LZ, nz, 3), st>>>(cs, lz, pZ, twz, LZ);
   }
   pass_y(Tsp, +1);
-  if (kx) {
+  if (ko) {
     const double2* spec = Tsp;
     void* args[] = {&nlines, &spec, &d_out, &twx, &scale};
-    if (e == cudaSuccess) e = launch(kx->c2r, gx, kx->threads, args, kx->smem[3], st);
+    if (e == cudaSuccess) e = launch(ko->c2r, grid_x(ko), ko->threads, args, ko->smem[3], st);
   } else {
-    k_noalloc_xinv<<<gx, 256, x_smem_of(nl, nx), st>>>(g, Tsp, d_out, p2, twx, scale, nl);
+    k_noalloc_xinv<<<grid_x(nullptr), 256, x_smem_of(nl, nx), st>>>(g, Tsp, d_out, p2, twx, scale, nl);
   }
   if (e != cudaSuccess) {
     cudaGetLastError();

@@ -399,7 +399,9 @@ long long ep_device_bytes(const ep_ctx* ctx);
  * (poten.f90:27-50).  d_in and d_out are real (nx,ny,nz) device arrays,
  * d_kernel the real half-spectrum table (nx/2+1,ny,nz) on the device;
  * stream is a cudaStream_t (NULL: the default stream).  The call is
- * asynchronous on that stream.
+ * asynchronous on that stream.  d_in must be 16-byte aligned, d_kernel and
+ * d_out as any double (EP_ERR_INVALID_ARG otherwise, before any device work);
+ * a 16-byte aligned d_out is faster.
  *
  * Scratch lives in one fixed device array of the library (4.3 MB, held on
  * every GPU that loads the library until the process exits), so:
