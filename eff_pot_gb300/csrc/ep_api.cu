@@ -569,7 +569,10 @@ static void parabolas(const double* f, int npot, double h, int at, std::vector<d
 
 // Replaces the device tables by tabs[0..2] (NULL: none) of npot + 2 entries
 // each: in the D state d_potpi, d_potdel, d_potsigdel; in the P state the
-// parabolas of tabs[0] and tabs[1] and their FP32 copies.
+// parabolas of tabs[0] and tabs[1] and their FP32 copies.  The copies go on the
+// context's stream, which does not wait for the legacy one (a pageable
+// cudaMemcpy returns once staged), and are waited for before the host's copies
+// go.
 static int upload_tables(ep_ctx* c, const double* const tabs[3], int npot, double delinter) {
   cudaSetDevice(c->cfg.device);
   ImpState& m = c->imp;
@@ -590,26 +593,29 @@ static int upload_tables(ep_ctx* c, const double* const tabs[3], int npot, doubl
       *d = nullptr;
       return fail(c, EP_ERR_OOM, "table allocation failed");
     }
-    if (cudaMemcpy(*d, h, n, cudaMemcpyHostToDevice) != cudaSuccess)
+    if (cudaMemcpyAsync(*d, h, n, cudaMemcpyHostToDevice, c->st) != cudaSuccess)
       return fail(c, EP_ERR_CUDA, "table upload failed");
     return EP_OK;
   };
   const size_t n = (size_t)npot + 2;
-  int r;
-  if (c->cfg.state == EP_STATE_D) {
-    for (int i = 0; i < 3; ++i)
-      if (tabs[i] && (r = put((void**)dst[i], tabs[i], n * sizeof(double)))) return r;
-    return EP_OK;
-  }
   const double rmax = (npot - 1) * delinter, h = rmax / (npot - 1);
-  std::vector<double> coef(2 * n * 8, 0.0);
-  std::vector<float> tf(n);
-  for (int i = 0; i < 2; ++i) {
-    parabolas(tabs[i], npot, h, 3 * i, coef);
-    for (size_t k = 0; k < n; ++k) tf[k] = (float)tabs[i][k];
-    if ((r = put((void**)dstf[i], tf.data(), n * sizeof(float)))) return r;
+  std::vector<double> coef;
+  std::vector<float> tf[2];
+  int r = EP_OK;
+  if (c->cfg.state == EP_STATE_D) {
+    for (int i = 0; i < 3 && !r; ++i)
+      if (tabs[i]) r = put((void**)dst[i], tabs[i], n * sizeof(double));
+  } else {
+    coef.assign(2 * n * 8, 0.0);
+    for (int i = 0; i < 2 && !r; ++i) {
+      parabolas(tabs[i], npot, h, 3 * i, coef);
+      tf[i].assign(tabs[i], tabs[i] + n);
+      r = put((void**)dstf[i], tf[i].data(), n * sizeof(float));
+    }
+    if (!r) r = put((void**)&m.d_coef, coef.data(), coef.size() * sizeof(double));
   }
-  return put((void**)&m.d_coef, coef.data(), coef.size() * sizeof(double));
+  const bool done = cudaStreamSynchronize(c->st) == cudaSuccess;
+  return r || done ? r : fail(c, EP_ERR_CUDA, "table upload failed");
 }
 
 int ep_set_impurity_tables(ep_ctx* c, const double* potpi, const double* potdel, int npot, double delinter,
