@@ -547,23 +547,16 @@ int ep_set_impurity_potentials(ep_ctx* c, const ep_potential* pi, const ep_poten
   return ep_set_impurity_tables(c, tp.data(), td.data(), npot, del, sigma->umax);
 }
 
-// The parabolas of update() (potenimp.f90:588-632) through f(i0-1), f(i0),
-// f(i0+1) for every i0 and for both of its branches (r below the node i0 first,
-// then above), with its coefficients aa, bb, cc of r: entries at
-// ((branch * (npot + 2) + i0) * 8 + at).
+// The parabola of update() (potenimp.f90:588-632) through f(i0-1), f(i0),
+// f(i0+1) about the node i0, f0 + d (b + aa d), for every i0: entries at
+// (i0 * 8 + at).
 static void parabolas(const double* f, int npot, double h, int at, std::vector<double>& coef) {
-  const double c1oh = 1.0 / h, c1o2h2 = c1oh * c1oh * 0.5;
-  for (int branch = 0; branch < 2; ++branch) {
-    for (int i0 = 1; i0 <= npot; ++i0) {
-      const bool lo = branch == 0;
-      const double r0 = (i0 - 1) * h, f0 = f[i0], f1 = f[lo ? i0 - 1 : i0 + 1], f2 = f[lo ? i0 + 1 : i0 - 1];
-      const double aa = (f2 - 2.0 * f0 + f1) * c1o2h2;
-      const double bb = ((lo ? f2 : f1) - f0) * c1oh - aa * (2.0 * r0 + h);
-      double* o = coef.data() + ((size_t)branch * (npot + 2) + i0) * 8 + at;
-      o[0] = aa;
-      o[1] = bb;
-      o[2] = f0 - r0 * (bb + r0 * aa);
-    }
+  const double c1oh = 1.0 / h;
+  for (int i0 = 1; i0 <= npot; ++i0) {
+    double* o = coef.data() + (size_t)i0 * 8 + at;
+    o[0] = f[i0];
+    o[1] = 0.5 * (f[i0 + 1] - f[i0 - 1]) * c1oh;
+    o[2] = 0.5 * ((f[i0 + 1] - f[i0]) - (f[i0] - f[i0 - 1])) * c1oh * c1oh;
   }
 }
 
@@ -606,7 +599,7 @@ static int upload_tables(ep_ctx* c, const double* const tabs[3], int npot, doubl
     for (int i = 0; i < 3 && !r; ++i)
       if (tabs[i]) r = put((void**)dst[i], tabs[i], n * sizeof(double));
   } else {
-    coef.assign(2 * n * 8, 0.0);
+    coef.assign(n * 8, 0.0);
     for (int i = 0; i < 2 && !r; ++i) {
       parabolas(tabs[i], npot, h, 3 * i, coef);
       tf[i].assign(tabs[i], tabs[i] + n);

@@ -63,8 +63,8 @@ struct ImpState {
     erriv = 0;
   }
   // interpolation tables (module interpol), FP64 on the device
-  // P state: d_coef, the parabolas of V_Pi and V_Sigma - V_Pi per interval and
-  // side (ImpTable).  D state: d_potdel = V_Delta, d_potpi = V_Pi - V_Delta,
+  // P state: d_coef, the parabolas of V_Pi and V_Sigma - V_Pi per node
+  // (ImpTable).  D state: d_potdel = V_Delta, d_potpi = V_Pi - V_Delta,
   // d_potsigdel = V_Sigma - V_Delta.
   int npot = 0;
   double delinter = 0, umax_sigma = 9.674836e3, umax_pi = 0.0;

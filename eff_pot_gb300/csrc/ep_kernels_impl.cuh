@@ -75,52 +75,42 @@ EP_DEV void columns(const Geo& g, const ColGrid& cg, Setup&& setup, Body&& body,
   }
 }
 
-// V_Pi and the P-state Delta of updatepoten at |x - r_imp|^2 = rr2, from the
-// parabolas of update() (potenimp.f90:588-632) tabulated per interval and side
-// (upload_tables).  r and 1 / r^2 come from one reciprocal square root with a
-// correction of r; where r / h falls within 1e-5 of a switch of the parabola
-// (the next interval, or the other side of a node), r <= 1e-3 or the table's
-// end, the root and the quotients are taken as update() takes them, so the
-// interval is the one it takes.
+// V_Pi and the P-state Delta of updatepoten at |x - r_imp|^2 = rr2.  update()
+// (potenimp.f90:588-632) evaluates, in both of its branches, the parabola
+// through f(i0-1), f(i0), f(i0+1); it is tabulated per node i0 (upload_tables)
+// about the node r0 = (i0-1) h.  Coefficients about r = 0, as update() forms
+// them, cancel beside a cut-off core (1000 K over h = 0.01 A: aa r^2 = 5e7, 1e-8
+// K of rounding at every point within h of it: the excited-impurity job's
+// energies and psi were off by 4e-14, and by 2.6e-14 with another order of
+// operations).  i0 is update()'s: where r / h falls within 1e-5 of a switch of
+// the parabola, or r <= 1e-3 or the table's end, it is taken with update()'s
+// quotient.
 struct ImpTable {
-  const double* coef;  // [2][npot + 2][8]: aa, bb, cc of V_Pi, then of V_Sigma - V_Pi
+  const double* coef;  // [npot + 2][8]: f0, slope and curvature / 2 of V_Pi, then of V_Sigma - V_Pi
   int npot;
   double h, rh;        // spacing and its reciprocal
   double umax_sigma;
 };
-// 1 / sqrt(x) for normal x > 0: the approximate root instruction (about 2^-20)
-// and one third-order correction y += y e (1/2 + 3/8 e), e = 1 - x y^2 (left:
-// 5/16 e^3, below 2^-57), six FP64-pipe operations.
-EP_DEV double fast_rsqrt(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x * y, y, 1.0);
-  return fma(y * e, fma(e, 0.375, 0.5), y);
-}
 EP_DEV void imp_field(const ImpTable& t, double rr2, double& vp, double& dl) {
-  const double rs = fast_rsqrt(rr2);
-  double r = rr2 * rs;
-  r = fma(fma(-r, r, rr2), 0.5 * rs, r);
+  const double r = sqrt(rr2);
   const double q = fma(r, t.rh, 1.5);
   int i0 = (int)q;
+  double di = (double)i0;
   // compared in FP32 and, for rr2 > 1.1e-6, by the exponent word (an FP64
   // comparison is an FP64-pipe operation)
-  const float fr = (float)(q - (double)i0);
-  bool lo = fr < 0.5f;
-  const bool plain = __double2hiint(rr2) > 0x3eb27476 && fr > 1e-5f && fr < 1.0f - 1e-5f && fabsf(fr - 0.5f) > 1e-5f &&
-                     i0 < t.npot;
+  const float fr = (float)(q - di);
+  const bool plain = __double2hiint(rr2) > 0x3eb27476 && fr > 1e-5f && fr < 1.0f - 1e-5f && i0 < t.npot;
   if (!plain) {
-    r = sqrt(rr2);
-    i0 = (int)(1.5 + r / t.h);
-    i0 = min(max(i0, 1), t.npot);
-    lo = r < (i0 - 1) * t.h;
+    i0 = min(max((int)(1.5 + r / t.h), 1), t.npot);
+    di = (double)i0;
   }
-  const double2* c = reinterpret_cast<const double2*>(t.coef + ((lo ? 0 : t.npot + 2) + i0) * 8);
+  const double2* c = reinterpret_cast<const double2*>(t.coef + i0 * 8);
   const double2 c0 = __ldg(c), c1 = __ldg(c + 1), c2 = __ldg(c + 2);
-  vp = r * (c0.x * r + c0.y) + c1.x;
-  dl = r * (c1.y * r + c2.x) + c2.y;
-  if (plain) dl *= rs * rs;
-  else dl = r > 1e-3 ? dl / rr2 : t.umax_sigma;
+  const double d = fma(1.0 - di, t.h, r);
+  vp = d * (c1.x * d + c0.y) + c0.x;
+  dl = d * (c2.y * d + c2.x) + c1.y;
+  if (plain || r > 1e-3) dl = dl / rr2;
+  else dl = t.umax_sigma;
 }
 
 // A double as a field value.  The double-float split rounds to 24 bits in the
@@ -138,10 +128,11 @@ template <> EP_DEV dfloat to_field<dfloat>(double d) {
   return dfloat(__uint_as_float(m | ((unsigned)(rb >> 32) & 0x80000000u)), (float)(d - __longlong_as_double(rb)));
 }
 
-// The field of the P-state impurity.  Bound by the FP64 pipe (about 45
-// operations a point with double-float stores, 35 in FP64; the table
-// arithmetic, a division by h and one by r^2 per point were 120): 96 x 160 x
-// 192 double-float 623 -> 292 us.
+// The field of the P-state impurity.  Bound by the FP64 pipe (about 50
+// operations a point with double-float stores, 44 in FP64; the table
+// arithmetic, coordinates and two divisions per point were 120): 96 x 160 x 192
+// double-float 559 -> 366 us, 64 x 64 x 80 FP64 69 -> 44.  With r and 1 / r^2
+// from one reciprocal root it took 320 and 37 us, but 1 / r^2 lost two bits.
 template <class T>
 __global__ void __launch_bounds__(256) k_potenimp(Geo g, ColGrid cg, double xmax, double ymax, double zmax, double hx,
                                                   double hy, double hz, double r0, double r1, double r2, ImpTable t,
