@@ -357,11 +357,13 @@ EP_DEV float fmul1(float a, float b) { return a * b; }
 // den Delta and den V_Pi (1, y, y^2) and the column's x and z factors are
 // applied once per column: seven products and seven compensated sums a point
 // in the fields' own arithmetic (FP32; pairs of FP32 values in double-float;
-// FP64).  In double-float the products' 2^-45 is below the fields' own
-// rounding, and the FP64 conversions, products and sums of the one-point form
-// (about 120 operations a point on the FP64 pipe) go: 96 x 160 x 192 896 ->
-// 46 us; FP64 64 x 64 x 80 360 -> 123 us; FP32 256 x 256 x 320
-// 168 -> 120 us (memory: seven fields read).  MOM = false: the force alone
+// FP64).  In double-float a thread's sums are pairs, whose roundings (2^-46 of a
+// product, 2^-49 of a sum) average out over points and threads, and the block's
+// are FP64: the force is within 5e-17 of its terms' magnitudes, the moments
+// within 1e-16 (2e-16 with the block's sums in pairs too).  The FP64
+// conversions, products and sums of the one-point form (about 120 operations a
+// point on the FP64 pipe) go: 96 x 160 x 192 896 -> 54 us; FP64 64 x 64 x 80 361
+// -> 111 us; FP32 256 x 256 x 320 168 -> 120 us (memory: seven fields read).  MOM = false: the force alone
 // (three sums, four fields read).
 template <class T, bool MOM>
 __global__ void __launch_bounds__(256) k_impmoments(Geo g, ColGrid cg, const T* __restrict__ den,
@@ -382,7 +384,8 @@ __global__ void __launch_bounds__(256) k_impmoments(Geo g, ColGrid cg, const T* 
   for (int i = threadIdx.x + 32 * threadIdx.y; i < cg.rows; i += 32 * blockDim.y)
     ys[i] = T(coord(ymax, hy, y0 + i) - r1);
   __syncthreads();
-  Acc<T> acc[MOM ? 9 : 3];
+  constexpr int NQ = MOM ? 9 : 3;
+  Acc<T> acc[NQ];
   Acc<T> sv, s0, s1, s2;  // along the column: den V_Pi and den Delta (1, y, y^2)
   T xx = T(0), zz = T(0);
   bool fz = false;
@@ -421,7 +424,14 @@ __global__ void __launch_bounds__(256) k_impmoments(Geo g, ColGrid cg, const T* 
         acc[8].add(mul(zz, Dz));
         }
       });
-  block_reduce_store_acc<MOM ? 9 : 3>(acc, partials);
+  if constexpr (std::is_same<T, dfloat>::value) {
+    double tot[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) tot[q] = acc[q].get();
+    block_reduce_store_sums<NQ>(tot, partials);
+  } else {
+    block_reduce_store_acc<NQ>(acc, partials);
+  }
 }
 
 // Sum of |psi|^2 (block partials).
@@ -489,21 +499,29 @@ EP_DEV double one_plus_tanh(const Phys& ph, double dn) {
   }
   return 1.0 + tanh(ph.beta * (dn - ph.den_m));
 }
+// The same in pairs (an FP32 argument, whose rounding of 2 beta den_m alone is
+// 4e-7 of e, put 3.7e-7 into every sum; FP64's 1 + tanh leaves 3e-8).
 template <class T>
 EP_DEV dfloat one_plus_tanh_f(const Phys& ph, T dn) {
-  const float b2 = 2.0f * ph.f.beta, y = fmaf(b2, (float)dn, -b2 * ph.f.den_m);
-  if (y < -25.0f) return dfloat(2.0f * expf(y));
+  const dfloat y = dfloat(2.0f, 0.0f) * ph.d.beta * (dfloat(dn) - ph.d.den_m);
+  if (y.hi < -25.0f) {
+    const dfloat e = dd_exp(y);
+    return dfloat(2.0f, 0.0f) * (e - e * e);  // 2 e / (1 + e)
+  }
   return dfloat(1.0 + tanh(ph.beta * (dbl(dn) - ph.den_m)));
 }
 
 // Energy integrals.  W: the arithmetic of the terms (W = double: FP64; W =
 // dfloat: pairs of FP32 values, exact products of FP32 fields, 2^-45 for
-// double-float ones, summed in FP32 pairs).  The FP64 form of every engine was
-// bound by the FP64 pipe (about 380 operations a point: conversions, tanh,
-// eight Neumaier sums); FP32 fields in pairs leave the pipe to a U+ that
-// is no Morse potential (its distance and pair potential).  128^3, impurity with a Morse U+: FP32 1142 ->
-// 169 us, double-float 1333 -> 272, FP64 1260 -> 953 (64^3: 426
-// -> 151).  The caller falls back to W = double where the pairs' FP32
+// double-float ones, summed in FP32 pairs by a thread and in FP64 by a block:
+// each sum within about 1e-16 of its terms' magnitudes, as the FP64 form, but
+// the Morse U+ of FP32 fields, 3e-13; the two powers of the coarse-grained
+// density apart, whose FP64 coefficients cancel).  The FP64 form of every
+// engine was bound by the FP64 pipe (about 380 operations a point:
+// conversions, tanh, eight Neumaier sums); FP32 fields in pairs leave the pipe
+// to a U+ that is no Morse potential (its distance and pair potential).
+// 128^3, impurity with a Morse U+: FP32 1133 -> 174 us, double-float 1333 ->
+// 286, FP64 1260 -> 953 (64 x 64 x 80: 460 -> 200).  The caller falls back to W = double where the pairs' FP32
 // range does not hold the sums.
 template <class T, class W>
 __global__ void __launch_bounds__(256) k_energy(Geo g, ColGrid cg, const __grid_constant__ FdW<T> fd, Phys ph, const C2<T>* __restrict__ psi,
@@ -517,7 +535,7 @@ __global__ void __launch_bounds__(256) k_energy(Geo g, ColGrid cg, const __grid_
                                                 double zexc, const __grid_constant__ PotDev vplus, int impurity,
                                                 double* __restrict__ partials) {
   constexpr bool D64 = std::is_same<W, double>::value;
-  Acc<W> acc[8];
+  Acc<W> acc[D64 ? 8 : 9];  // pairs: n cg^2 and, as the ninth, n cg^3
   const bool otc = ph.core == 1;
   // FP32 fields: a Morse U+ in pairs of FP32 values (2^-36 and better; in FP64
   // its root and exponential were 200 us of the 255 at 128^3)
@@ -590,7 +608,9 @@ __global__ void __launch_bounds__(256) k_energy(Geo g, ColGrid cg, const __grid_
           acc[0].add(wmul(dz.x, dz.x));
           acc[0].add(wmul(dz.y, dz.y));
           acc[1].add(wmul(lj, dn));
-          acc[2].add(wmul(wmul(wmul(cg_, cg_), dn), ph.d.a0 + wmul(ph.d.a1, cg_)));
+          const dfloat nc2 = wmul(wmul(cg_, cg_), dn);
+          acc[2].add(nc2);
+          acc[8].add(wmul(nc2, cg_));
           if (otc)
             acc[3].add(wmul((wmul(dxd[p], ix_[p]) + wmul(dyd[p], iy_[p])) + wmul(dzd[p], iz_[p]), falfs[p]));
           acc[4].add(wmul(one_plus_tanh_f(ph, dn), dn));
@@ -615,7 +635,15 @@ __global__ void __launch_bounds__(256) k_energy(Geo g, ColGrid cg, const __grid_
         }
       },
       [] {});
-  block_reduce_store_acc<8>(acc, partials);
+  if constexpr (D64) {
+    block_reduce_store_acc<8>(acc, partials);
+  } else {
+    double tot[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) tot[q] = acc[q].get();
+    tot[2] = 0.5 * ph.cp4 * tot[2] + (1.0 / 3.0) * ph.cpp4 * acc[8].get();
+    block_reduce_store_sums<8>(tot, partials);
+  }
 }
 
 // ---------------------------------------------------------------------------
