@@ -31,6 +31,7 @@ struct StepGraph {
   // buffers when the capture began (the replay is valid at that phase only)
   int nsteps = 1;
   std::vector<std::array<const void*, 7>> sig0;
+  bool asked = false;  // a single full step has been wanted before (graph_steps)
   void reset() {
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
@@ -46,8 +47,9 @@ struct StepGraph {
 };
 
 struct ep_ctx {
-  StepGraph graph;
-  StepGraph graphk;  // one rotation period of steps
+  StepGraph graph;   // a lean step
+  StepGraph graphf;  // a full step
+  StepGraph graphk;  // one rotation period of steps, the last of them full
   int use_graphs = 1;  // 0 direct launches, 1 step graphs, 2 multi-step graphs
   ep_config cfg{};
   cudaStream_t st = nullptr;
@@ -62,8 +64,9 @@ struct ep_ctx {
 };
 
 struct ep_batch {
-  StepGraph graph;
-  StepGraph graphk;  // one rotation period of steps
+  StepGraph graph;   // a lean step
+  StepGraph graphf;  // a full step
+  StepGraph graphk;  // one rotation period of steps, the last of them full
   int use_graphs = 1;  // 0 direct launches, 1 step graphs, 2 multi-step graphs
   std::vector<ep_ctx*> ctx;
   cudaStream_t st = nullptr;
@@ -275,7 +278,13 @@ int capture_steps(StepGraph& G, const std::vector<ep_ctx*>& cs, cudaStream_t st,
     for (size_t i = 0; i < n && !r; ++i) {
       ep_ctx* c = cs[i];
       const long long l0 = c->prof.launches;
-      r = dispatch(c, [&](auto& e) -> int { return e.steppc(dt, nullptr); });
+      r = dispatch(c, [&](auto& e) -> int {
+        const bool lean = e.lean;
+        e.lean = lean && p < P - 1;
+        const int q = e.steppc(dt, nullptr);
+        e.lean = lean;
+        return q;
+      });
       G.launches[i] += c->prof.launches - l0;
     }
   }
@@ -313,35 +322,62 @@ int replay_steps(StepGraph& G, const std::vector<ep_ctx*>& cs, cudaStream_t st) 
   return EP_OK;
 }
 
-// ng graph-eligible (and lean) steps of every context of cs: whole rotation periods
-// from the multi-step graph Gk (captured at the first phase that needs it),
-// the rest -- realignment and remainder -- as single replayed steps of G1.
-int graph_steps(StepGraph& G1, StepGraph& Gk, const std::vector<ep_ctx*>& cs, cudaStream_t st, ep_batch* b,
-                double dt, int ng, int mode) {
-  int s = 0, r;
+// The graphs of one context or batch.
+struct StepGraphs {
+  StepGraph &lean, &full, &period;
+};
+
+// ng graph-eligible steps of every context of cs: whole rotation periods from
+// the multi-step graph (captured at the first phase that needs it), the rest --
+// realignment and remainder -- as single replayed steps.  All are lean (the
+// period's last one apart, so that a run may end with it), but with last_full
+// the ng-th, whose fields the caller may read.  done: the steps made; the ng-th
+// is left to the caller the first time a single full step is wanted (its
+// capture costs several direct steps, and most callers run once; a loop over
+// run(2, NULL) at 32^3 took 99 us a step with a direct last one, 70 with it
+// replayed).
+int graph_steps(StepGraphs G, const std::vector<ep_ctx*>& cs, cudaStream_t st, ep_batch* b, double dt, int ng,
+                bool last_full, int mode, int& done) {
+  const LeanSteps lean(cs);
+  int& s = done;
+  int r;
+  s = 0;
   auto single = [&]() -> int {
-    if (!graph_valid(G1, cs)) return capture_step(G1, cs, st, b, dt);
-    return replay_step(G1, cs, st, dt);
+    if (!graph_valid(G.lean, cs)) return capture_step(G.lean, cs, st, b, dt);
+    return replay_step(G.lean, cs, st, dt);
   };
+  const int singles = ng - (last_full ? 1 : 0);  // lean single steps end here
   const int P = mode >= 2 ? common_period(cs) : 0;
   if (P >= 2 && ng >= P) {
-    if (graph_valid(Gk, cs))
-      while (s < ng && !at_phase(Gk, cs)) {
+    if (graph_valid(G.period, cs))
+      while (s < singles && !at_phase(G.period, cs)) {
         if ((r = single())) return r;
         ++s;
       }
     if (ng - s >= P) {
-      if (!graph_valid(Gk, cs) || !at_phase(Gk, cs)) {
-        if ((r = capture_steps(Gk, cs, st, b, dt, P))) return r;
+      if (!graph_valid(G.period, cs) || !at_phase(G.period, cs)) {
+        if ((r = capture_steps(G.period, cs, st, b, dt, P))) return r;
         s += P;
       }
       for (; ng - s >= P; s += P)
-        if ((r = replay_steps(Gk, cs, st))) return r;
+        if ((r = replay_steps(G.period, cs, st))) return r;
     }
   }
-  for (; s < ng; ++s)
+  for (; s < singles; ++s)
     if ((r = single())) return r;
-  return EP_OK;
+  if (s == ng) return EP_OK;
+  if (!graph_valid(G.full, cs)) {
+    if (!G.full.asked) {
+      G.full.asked = true;
+      return EP_OK;
+    }
+    lean.set(false);
+    r = capture_step(G.full, cs, st, b, dt);
+  } else {
+    r = replay_step(G.full, cs, st, dt);
+  }
+  if (!r) ++s;
+  return r;
 }
 
 }  // namespace
@@ -498,6 +534,7 @@ int ep_destroy(ep_ctx* c) {
   cudaSetDevice(c->cfg.device);
   if (c->st) cudaStreamSynchronize(c->st);
   c->graph.reset();
+  c->graphf.reset();
   c->graphk.reset();
   if (c->e64) { c->e64->release(); delete c->e64; }
   if (c->e32) { c->e32->release(); delete c->e32; }
@@ -793,18 +830,16 @@ int ep_steppc(ep_ctx* c, double dt, ep_step_errors* err) {
 int ep_run(ep_ctx* c, int nsteps, double dt, ep_run_stats* stats) {
   if (!c || nsteps < 0) return EP_ERR_INVALID_ARG;
   const std::vector<ep_ctx*> one{c};
-  int s0 = 0;
-  // every step but the last: no statistics, and no field of it outlives it
-  const int ng = nsteps - 1;
-  if (ng > 0) {
+  int s0 = 0, r;
+  const int ng = nsteps - (stats ? 1 : 0);  // steps that need no host statistics
+  if (ng >= 2 && graph_eligible(c) &&
+      (r = graph_steps({c->graph, c->graphf, c->graphk}, one, c->st, nullptr, dt, ng, !stats, c->use_graphs, s0)))
+    return r;
+  if (s0 < nsteps - 1) {
+    // no field of a step before the last outlives the next one
     const LeanSteps lean(one);
-    int r;
-    if (ng >= 2 && graph_eligible(c)) {
-      if ((r = graph_steps(c->graph, c->graphk, one, c->st, nullptr, dt, ng, c->use_graphs))) return r;
-      s0 = ng;
-    }
     r = dispatch(c, [&](auto& e) -> int {
-      for (; s0 < ng; ++s0)
+      for (; s0 < nsteps - 1; ++s0)
         if (int q = e.steppc(dt, nullptr)) return q;
       return EP_OK;
     });
@@ -812,9 +847,9 @@ int ep_run(ep_ctx* c, int nsteps, double dt, ep_run_stats* stats) {
   }
   return dispatch(c, [&](auto& e) -> int {
     ep_step_errors se{};
-    if (nsteps > 0) {
-      int r = e.steppc(dt, stats ? &se : nullptr);
-      if (r) return r;
+    if (s0 < nsteps) {
+      int q = e.steppc(dt, stats ? &se : nullptr);
+      if (q) return q;
     }
     if (stats) {
       stats->errHe = se.errHe;
@@ -877,6 +912,7 @@ int ep_batch_destroy(ep_batch* b) {
   if (!b) return EP_ERR_INVALID_ARG;
   if (b->st) cudaStreamSynchronize(b->st);
   b->graph.reset();
+  b->graphf.reset();
   b->graphk.reset();
   for (ep_ctx* c : b->ctx) ep_destroy(c);
   cudaSetDevice(b->device);
@@ -900,15 +936,13 @@ int ep_batch_run(ep_batch* b, int nsteps, double dt, ep_run_stats* stats) {
   cudaSetDevice(b->device);
   batch_join(b);  // work the caller left on the instance streams comes first
   int s0 = 0;
-  // every step but the last: no statistics, and no field of it outlives it
-  const int ng = nsteps - 1;
+  const int ng = nsteps - (stats ? 1 : 0);  // steps that need no host statistics
   bool eligible = b->use_graphs > 0 && ng >= 2;
   for (ep_ctx* c : b->ctx) eligible = eligible && graph_eligible(c);
   if (eligible) {
-    const LeanSteps lean(b->ctx);
     int r;
-    if ((r = graph_steps(b->graph, b->graphk, b->ctx, b->st, b, dt, ng, b->use_graphs))) return r;
-    s0 = ng;
+    if ((r = graph_steps({b->graph, b->graphf, b->graphk}, b->ctx, b->st, b, dt, ng, !stats, b->use_graphs, s0)))
+      return r;
   }
   batch_fork(b);
   // step-major interleaving so the instances' kernels overlap
