@@ -1395,11 +1395,15 @@ int Engine<T>::autotune(std::string* report) {
     float fin = 0.f;
     if ((r = timed(fin))) goto done;
     if (report) {
-      char buf[256];
-      snprintf(buf, sizeof buf,
-               "poten %.3f -> %.3f ms; X1..X4 %dx%d %dx%d %dx%d %dx%d (lines x threads), Y %d x %d, Z %d x %d", base,
-               fin, shp.xnl[0], shp.xthr[0], shp.xnl[1], shp.xthr[1], shp.xnl[2], shp.xthr[2], shp.xnl[3],
-               shp.xthr[3], shp.ylt, shp.ythr, shp.zlt, shp.zthr);
+      char buf[160], xs[80], ys[24], zs[24];
+      snprintf(xs, sizeof xs, "%dx%d %dx%d %dx%d %dx%d", shp.xnl[0], shp.xthr[0], shp.xnl[1], shp.xthr[1], shp.xnl[2],
+               shp.xthr[2], shp.xnl[3], shp.xthr[3]);
+      snprintf(ys, sizeof ys, "%dx%d", shp.ylt, shp.ythr);
+      snprintf(zs, sizeof zs, "%dx%d", shp.zlt, shp.zthr);
+      // axes whose length has kernels of its own ignore the shapes
+      const char* own = "its length's kernels";
+      snprintf(buf, sizeof buf, "poten %.3f -> %.3f ms; lines x threads: X1..X4 %s, Y %s, Z %s", base, fin,
+               xw_kernels<T>(g.nx / 2) ? own : xs, yz_kernels<T>(g.ny) ? own : ys, yz_kernels<T>(g.nz) ? own : zs);
       *report = buf;
     }
   }
