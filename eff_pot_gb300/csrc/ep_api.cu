@@ -31,7 +31,7 @@ struct StepGraph {
   // buffers when the capture began (the replay is valid at that phase only)
   int nsteps = 1;
   std::vector<std::array<const void*, 7>> sig0;
-  bool asked = false;  // a single full step has been wanted before (graph_steps)
+  int asked = 0;  // how often a single full step has been wanted (graph_steps)
   void reset() {
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
@@ -331,11 +331,12 @@ struct StepGraphs {
 // the multi-step graph (captured at the first phase that needs it), the rest --
 // realignment and remainder -- as single replayed steps.  All are lean (the
 // period's last one apart, so that a run may end with it), but with last_full
-// the ng-th, whose fields the caller may read.  done: the steps made; the ng-th
-// is left to the caller the first time a single full step is wanted (its
-// capture costs several direct steps, and most callers run once; a loop over
-// run(2, NULL) at 32^3 took 99 us a step with a direct last one, 70 with it
-// replayed).
+// the ng-th, whose fields the caller may read.  done: the steps made; a step
+// whose graph would be replayed once is left to the caller the first three
+// times: a capture costs several direct steps, which callers of a few runs
+// never get back (the 42-step bench lost 0.5 % of its FP64 refinement), but a
+// loop over run(2, NULL) at 32^3 takes 99 us a step with direct ones and 63
+// replayed.
 int graph_steps(StepGraphs G, const std::vector<ep_ctx*>& cs, cudaStream_t st, ep_batch* b, double dt, int ng,
                 bool last_full, int mode, int& done) {
   const LeanSteps lean(cs);
@@ -347,6 +348,7 @@ int graph_steps(StepGraphs G, const std::vector<ep_ctx*>& cs, cudaStream_t st, e
     return replay_step(G.lean, cs, st, dt);
   };
   const int singles = ng - (last_full ? 1 : 0);  // lean single steps end here
+  if (singles == 1 && !graph_valid(G.lean, cs) && ++G.full.asked < 4) return EP_OK;
   const int P = mode >= 2 ? common_period(cs) : 0;
   if (P >= 2 && ng >= P) {
     if (graph_valid(G.period, cs))
@@ -367,10 +369,7 @@ int graph_steps(StepGraphs G, const std::vector<ep_ctx*>& cs, cudaStream_t st, e
     if ((r = single())) return r;
   if (s == ng) return EP_OK;
   if (!graph_valid(G.full, cs)) {
-    if (!G.full.asked) {
-      G.full.asked = true;
-      return EP_OK;
-    }
+    if (++G.full.asked < 4) return EP_OK;
     lean.set(false);
     r = capture_step(G.full, cs, st, b, dt);
   } else {
